@@ -349,6 +349,11 @@ int JMS_NnMseLoss(const float* out, const float* target, float* dout, float* los
  * BF16 copy to p_bf16 when given. */
 int JMS_NnAdam(float* p, const float* g, float* m, float* v, void* p_bf16, int n, float lr, float b1, float b2,
 	float eps, int step, void* stream);
+/* JMS_NnAdam on nset (at most 32) parameter tensors in one launch: host arrays
+ * of device pointers and sizes; p_bf16 may be NULL, or hold NULL for a tensor
+ * without a BF16 copy. */
+int JMS_NnAdamSet(int nset, float* const* p, const float* const* g, float* const* m, float* const* v,
+	void* const* p_bf16, const int* n, float lr, float b1, float b2, float eps, int step, void* stream);
 int JMS_NnCastBf16(const float* src, void* dst, long long n, void* stream);
 /* Surrogate inputs on the device: out [nconf][npos][nbins][win/pool][win/pool]
  * = the mean, over the object slices of each depth bin (nbins bins of

@@ -130,12 +130,16 @@ class SurrogateNet:
     def train_step(self, x, t, B: int, lr: float):
         loss = self.backward(x, t, B)
         self.step += 1
-        s = self._stream()
-        for k, p in enumerate(self.params):
-            pb = self.bf[k // 2].data_ptr() if (k % 2 == 0 and k // 2 < len(self.conv)) else None
-            e = self.L.JMS_NnAdam(p.data_ptr(), self.grads[k].data_ptr(), self.m[k].data_ptr(), self.v[k].data_ptr(),
-                                  pb, p.numel(), lr, 0.9, 0.999, 1e-8, self.step, s)
-            assert e == 0, e
+        n = len(self.params)
+        copies = [self.bf[k // 2] if (k % 2 == 0 and k // 2 < len(self.conv)) else None for k in range(n)]
+
+        def ptrs(ts):
+            return (C.c_void_p * n)(*[None if t is None else t.data_ptr() for t in ts])
+
+        e = self.L.JMS_NnAdamSet(n, ptrs(self.params), ptrs(self.grads), ptrs(self.m), ptrs(self.v), ptrs(copies),
+                                 (C.c_int * n)(*[p.numel() for p in self.params]), lr, 0.9, 0.999, 1e-8, self.step,
+                                 self._stream())
+        assert e == 0, e
         return loss
 
     def predict(self, x_all):
