@@ -609,9 +609,18 @@ int JmsB200::SetIncomingWaveGPU(const float* wav, bool bTranspose)
 	return 0;
 }
 
+// Wave pairs halve the CTAs of a launch, so they are taken where their column
+// tiles (8 columns of a pair) still reach every SM; results are the same bit
+// for bit either way.
+bool JmsB200::use_pairs(int nwave) const
+{
+	return nwave > 1 && prec_ == 0 && prow_ && pcol_ && prow_->row2 && pcol_->col2 &&
+		(long long)((nwave + 1) / 2) * ((nx_ + 7) / 8) >= 148;
+}
+
 int JmsB200::ensure_work(int nwave)
 {
-	const size_t need = (size_t)nwave * nx_ * ny_; // elements; the grid may change between setups
+	const size_t need = (size_t)(nwave > 1 ? nwave + (nwave & 1) : nwave) * nx_ * ny_; // room for whole pairs
 	if (need <= work_cap_ && d_work_) return 0;
 	dfree(d_work_);
 	work_cap_ = 0;
@@ -627,7 +636,7 @@ int JmsB200::ensure_partial(int nwave)
 	if (need <= partial_cap_ && d_partial_) return 0;
 	dfree(d_partial_);
 	partial_cap_ = 0;
-	if (post(cudaMalloc(&d_partial_, sizeof(float) * need), "partial sums")) return 1;
+	if (post(cudaMalloc(&d_partial_, sizeof(double) * need), "partial sums")) return 1;
 	partial_cap_ = need;
 	return 0;
 }
@@ -641,12 +650,16 @@ int JmsB200::run_slices(int nwave, int islc0, const int* var, float weight, cons
 	int nby, const int* plas, const int* d_plas_w, const int* d_mulw, int wave_pos)
 {
 	if (!prow_ || !pcol_) return 2;
-	if (ensure_work(nwave) || ensure_partial(nwave)) return 1;
 	const long long N = (long long)nx_ * ny_;
 	const bool b_dif = (imagedet_ & (DET_INTEGRATED | DET_DIFFRACTION | DET_WAVEFOURIER | DET_DIFFR_AVG | DET_WAVEF_AVG)) != 0;
 	const bool b_img = (imagedet_ & (DET_IMAGE | DET_WAVEREAL | DET_IMAGE_AVG | DET_WAVER_AVG)) != 0;
 	const bool single = (nwave == 1) && (d_bin == nullptr);
+	// several waves run in pairs where both plans have such passes (the images
+	// and channels of a run of one wave, and the tensor-core passes, are not
+	// among them)
+	const bool pairs = use_pairs(nwave);
 	const int ndet = (imagedet_ & DET_INTEGRATED) ? ndet_ : 0;
+	if (ensure_work(nwave) || ensure_partial(nwave)) return 1;
 	PassArgs base;
 	base.work = d_work_;
 	base.wstride = N;
@@ -676,7 +689,7 @@ int JmsB200::run_slices(int nwave, int islc0, const int* var, float weight, cons
 	}
 	cudaStream_t s = stream_;
 	if (base.ndet > 0) {
-		if (post(cudaMemsetAsync(d_partial_, 0, sizeof(float) * (size_t)nwave * ndetslc_ * ndet_ * base.nblk, s), "partials"))
+		if (post(cudaMemsetAsync(d_partial_, 0, sizeof(double) * (size_t)nwave * ndetslc_ * ndet_ * base.nblk, s), "partials"))
 			return 101;
 	}
 	auto plane_of = [&](int p) { return (p >= 0 && p <= nobjslc_) ? det_objslc_[p] : -1; };
@@ -693,7 +706,7 @@ int JmsB200::run_slices(int nwave, int islc0, const int* var, float weight, cons
 		p.ibty = ibty;
 		p.plane = b_dif ? plane_of(islc) : -1;
 		if (src_gap) { p.row_k1 = wav0_k1_; p.row_k2 = wav0_k2_; }
-		if (post(prow_->entry(p, s), "GPUMultislice entry")) return 101;
+		if (post((pairs ? prow_->entry2 : prow_->entry)(p, s), "GPUMultislice entry")) return 101;
 		launches_++;
 	}
 	// live Fourier rows (band of the propagator last applied; after the entry,
@@ -710,7 +723,7 @@ int JmsB200::run_slices(int nwave, int islc0, const int* var, float weight, cons
 		else c.mul = d_pgr_ + slcoffset_[st] + (long long)var[j] * npgx_ * npgy_;
 		c.npgx = npgx_;
 		c.npgy = npgy_;
-		c.plane = b_img ? plane_of(j) : -1;
+		c.plane = b_img && !pairs ? plane_of(j) : -1;
 		c.in_k1 = in_k1;
 		c.in_k2 = in_k2;
 		c.out_k1 = pro_k1_[ip];
@@ -726,7 +739,7 @@ int JmsB200::run_slices(int nwave, int islc0, const int* var, float weight, cons
 			if (post(launch_tc_col(c, prec_, d_tcerr_, s), "GPUMultislice column pass (tensor core)")) return 401;
 			tc_launches_++;
 		}
-		else if (post(pcol_->col(c, s), "GPUMultislice column pass")) return 401;
+		else if (post((pairs ? pcol_->col2 : pcol_->col)(c, s), "GPUMultislice column pass")) return 401;
 		if (timing_on_) { ev_col_.push_back(timed_event()); cudaEventRecord(ev_col_.back(), s); }
 		PassArgs r = four;
 		r.mul = d_pro_ + (long long)ip * N;
@@ -742,11 +755,11 @@ int JmsB200::run_slices(int nwave, int islc0, const int* var, float weight, cons
 			if (post(launch_tc_row(r, prec_, d_tcerr_, s), "GPUMultislice row pass (tensor core)")) return 601;
 			tc_launches_++;
 		}
-		else if (post(prow_->row(r, s), "GPUMultislice row pass")) return 601;
+		else if (post((pairs ? prow_->row2 : prow_->row)(r, s), "GPUMultislice row pass")) return 601;
 		if (timing_on_) { ev_row_.push_back(timed_event()); cudaEventRecord(ev_row_.back(), s); }
 		launches_ += 2;
 	}
-	if (b_img) { // exit plane image readout
+	if (b_img && !pairs) { // exit plane image readout
 		PassArgs c = real;
 		c.plane = plane_of(nobjslc_);
 		c.in_k1 = in_k1;
@@ -1020,13 +1033,15 @@ int JmsB200::Autotune(int nwave, int reps, float* ms_row, float* ms_col, int* ir
 	for (int i = 0; i < plan_count(nx_); i++) {
 		PassArgs p = base;
 		p.mul = d_pro_;
-		const float t = time_it(plan_get(nx_, i)->row, p);
+		const PlanOps* o = plan_get(nx_, i);
+		const float t = time_it(use_pairs(nwave) && o->row2 ? o->row2 : o->row, p);
 		if (t < tr) { tr = t; best_r = i; }
 	}
 	for (int i = 0; i < plan_count(ny_); i++) {
 		PassArgs p = base;
 		p.mul = d_pgr_;
-		const float t = time_it(plan_get(ny_, i)->col, p);
+		const PlanOps* o = plan_get(ny_, i);
+		const float t = time_it(use_pairs(nwave) && o->col2 ? o->col2 : o->col, p);
 		if (t < tc) { tc = t; best_c = i; }
 	}
 	cudaEventDestroy(e0);

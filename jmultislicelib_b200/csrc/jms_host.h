@@ -190,6 +190,7 @@ public:
 private:
 	int gpu_ready(int need) const { return (status_gpu_ & need) == need; }
 	int post(cudaError_t e, const char* where);
+	bool use_pairs(int nwave) const;   // passes over wave pairs for this many waves
 	int ensure_work(int nwave);
 	int ensure_partial(int nwave);
 	// d_mulw (with var == nullptr): per-slice per-wave grating offsets
@@ -235,7 +236,7 @@ private:
 	float2* d_twy_ = nullptr;
 	float2* d_work_ = nullptr;     // working waves [nwave][ny][nx]
 	size_t work_cap_ = 0;          // capacity in complex elements
-	float* d_partial_ = nullptr;   // per-CTA detector partial sums
+	double* d_partial_ = nullptr;  // per-CTA detector partial sums
 	size_t partial_cap_ = 0;
 	double* d_detint_ = nullptr;   // single-run integrated detectors [ndetslc][ndet]
 	double* d_shift_ = nullptr;    // per-wave offsets (scan)

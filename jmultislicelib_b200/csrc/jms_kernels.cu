@@ -51,20 +51,25 @@ cudaError_t launch_cv_combine(double* out, const double* g1, const double* gm, l
 	return cudaGetLastError();
 }
 
-// thread i = (position p, plane, detector) of n outputs; m = ndetslc * ndet
-// elements per wave; the waves of position p are p + k * step, k < nk
-__global__ void k_finalize(const float* __restrict__ partial, int n, int m, int nblk, int step, int nk, float weight,
-	double* det_int)
+// warp i = (position p, plane, detector) of n outputs; m = ndetslc * ndet
+// elements per wave; the waves of position p are p + k * step, k < nk.  The nk *
+// nblk terms go over the lanes, whose sums are added in a fixed order (one
+// thread walking them took 144 us for 16 x 64 terms of 2112 outputs: a chain of
+// dependent FP64 adds and loads).
+__global__ void __launch_bounds__(256) k_finalize(const double* __restrict__ partial, int n, int m, int nblk, int step,
+	int nk, float weight, double* det_int)
 {
-	const int i = blockIdx.x * blockDim.x + threadIdx.x;
+	const int i = (blockIdx.x * 256 + threadIdx.x) / 32, lane = threadIdx.x & 31;
 	if (i >= n) return;
 	const int pos = i / m, e = i - pos * m;
 	double s = 0.0;
 	for (int k = 0; k < nk; k++) {
-		const float* src = partial + ((long long)(pos + k * step) * m + e) * nblk;
-		for (int b = 0; b < nblk; b++) s += (double)src[b];
+		const double* src = partial + ((long long)(pos + k * step) * m + e) * nblk;
+		for (int b = lane; b < nblk; b += 32) s += src[b];
 	}
-	det_int[i] += (double)weight * s;
+	#pragma unroll
+	for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+	if (lane == 0) det_int[i] += (double)weight * s;
 }
 
 __global__ void k_gather_shift(double* __restrict__ sh_w, const double* __restrict__ sh, int npos, int nwave)
@@ -100,8 +105,7 @@ __global__ void k_offset(float2* out, const float2* __restrict__ wav0, int nx, i
 // plan table
 // ---------------------------------------------------------------------------
 static const PlanOps kPlans[] = {
-#define X(n_, pl_, name_) {n_, name_, &row_blocks_t<pl_>, &launch_entry_t<pl_>, &launch_row_t<pl_>, \
-	&launch_col_t<pl_>, &launch_exit_t<pl_>},
+#define X(n_, pl_, name_) plan_ops_t<pl_>(n_, name_),
 	JMS_PLANS(X)
 #undef X
 };
@@ -121,7 +125,7 @@ const PlanOps* plan_get(int n, int idx)
 	return nullptr;
 }
 
-cudaError_t launch_finalize(const float* partial, int nwave, int ndetslc, int ndet, int nblk, float weight,
+cudaError_t launch_finalize(const double* partial, int nwave, int ndetslc, int ndet, int nblk, float weight,
 	double* det_int, cudaStream_t s, int wave_pos)
 {
 	const int m = ndetslc * ndet;
@@ -129,7 +133,7 @@ cudaError_t launch_finalize(const float* partial, int nwave, int ndetslc, int nd
 	const int nk = wave_pos > 0 ? nwave / wave_pos : 1;
 	const int n = npos * m;
 	if (n <= 0) return cudaSuccess;
-	k_finalize<<<(n + 255) / 256, 256, 0, s>>>(partial, n, m, nblk, npos, nk, weight, det_int);
+	k_finalize<<<(n + 7) / 8, 256, 0, s>>>(partial, n, m, nblk, npos, nk, weight, det_int);
 	return cudaGetLastError();
 }
 

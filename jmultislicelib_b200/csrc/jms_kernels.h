@@ -23,8 +23,8 @@ namespace jms {
 constexpr int kMaxDet = 8;          // integrating detectors fused into one pass
 
 struct PassArgs {
-	float2* work = nullptr;         // [nwave][ny][nx] working waves
-	long long wstride = 0;          // elements between consecutive waves
+	float2* work = nullptr;         // [nwave][ny][nx] working waves, or [ceil(nwave / 2)][ny][nx] wave pairs
+	long long wstride = 0;          // elements between consecutive waves (or wave pairs)
 	int nx = 0, ny = 0, nwave = 0;
 	const float2* twx = nullptr;    // exp(-2 pi i k / nx), k < nx
 	const float2* twy = nullptr;    // exp(-2 pi i k / ny), k < ny
@@ -37,7 +37,7 @@ struct PassArgs {
 	float weight = 1.f;
 	int ndet = 0;                   // integrating detectors (0 = off)
 	const float* det = nullptr;     // [ndet][ny][nx], masks folded in
-	float* partial = nullptr;       // [nwave][ndetslc][ndet][nblk] per-CTA sums
+	double* partial = nullptr;      // [nwave][ndetslc][ndet][nblk] per-CTA sums
 	int nblk = 0;                   // row-pass CTAs per wave
 	long long chan_wstride = 0;     // per-wave stride of full-size channels (0 = one shared channel)
 	float* dif = nullptr;           // Fourier channels [ndetslc][ny][nx]
@@ -94,6 +94,11 @@ struct PlanOps {
 	cudaError_t (*row)(const PassArgs&, cudaStream_t);      // row pass
 	cudaError_t (*col)(const PassArgs&, cudaStream_t);      // column pass
 	cudaError_t (*exit)(const PassArgs&, cudaStream_t);     // exit column pass
+	// the passes over pairs of waves (PassArgs::work holds pairs; no channels
+	// or images), nullptr for a plan that has none
+	cudaError_t (*entry2)(const PassArgs&, cudaStream_t);
+	cudaError_t (*row2)(const PassArgs&, cudaStream_t);
+	cudaError_t (*col2)(const PassArgs&, cudaStream_t);
 };
 int plan_count(int n);
 const PlanOps* plan_get(int n, int idx);
@@ -113,7 +118,7 @@ cudaError_t launch_tc_col(const PassArgs& p, int prec, int* err, cudaStream_t s)
 // det_int[w][plane][d] += weight * sum_blk partial[w][plane][d][blk] (FP64);
 // with wave_pos > 0 the waves w = p + k wave_pos (k = 0, 1, ...) are summed
 // into position p, in that order (deterministic)
-cudaError_t launch_finalize(const float* partial, int nwave, int ndetslc, int ndet, int nblk, float weight,
+cudaError_t launch_finalize(const double* partial, int nwave, int ndetslc, int ndet, int nblk, float weight,
 	double* det_int, cudaStream_t s, int wave_pos = 0);
 
 // sh_w[w] = sh[w % npos] (4 doubles each), w < nwave: per-wave probe offsets

@@ -25,8 +25,19 @@
 // (split 2, split 1 with A = B, and split 1 with B > A on a row tile of B
 // threads per line) exchanges under warp barriers only, so the warps of a CTA
 // run their lines independently; column lines span the CTA's warps and take
-// CTA barriers.  Stage twiddles come from a shared copy (TwShared) where the
-// plan's table layout allows it.
+// CTA barriers.  Stage twiddles come from a shared copy (TwShared).
+//
+// A launch of many waves holds two of them per thread (cpair, jms_fft.cuh) in
+// packed arithmetic: 59 thread instructions per element of the column pass
+// against 84 with one wave.  Per 512-wave launch at 512^2 the
+// column pass takes 424 us against 505, the row pass 278 against 311 (16 warps
+// of 128 registers per SM against 32 of 64).  Without its wave loads and stores
+// the column pass still takes 377 us (449 with single waves): it is bound by
+// on-chip work, FMA pipe, shared memory and issue each at about 60 %, not by
+// DRAM (222 us for its bytes).  Measured slower: 8 x 8 x 8 lines (589 / 510 us),
+// 4 or 16 columns of pairs per tile (476, 604), fewer registers with spills
+// (513, 649), and the halves of one line as a pair in place of two waves
+// (440 / 328).
 #pragma once
 #include "jms_fft.cuh"
 #include "jms_kernels.h"
@@ -58,14 +69,14 @@ struct RowTile {
 	// warp barriers, and the warps of a CTA run their lines independently.
 	template <int P>
 	__host__ __device__ static constexpr bool warp_lines() { return 32 % (W > 0 ? W : P) == 0; }
-	// split 1 exchange S(line, k1, j), k1 < A, j < B, rows padded to B+1.  A
+	// split 1 exchange S(line, k1, j), k1 < A, j < B, rows of odd length.  A
 	// line's region has the same size for <A, B> and <B, A> (the forward and
 	// inverse exchanges), so with warp-local lines one line's inverse exchange
 	// never writes into another line's forward exchange.
 	template <int A, int B>
-	__host__ __device__ static constexpr int pad_line() { return A * (B + 1) > B * (A + 1) ? A * (B + 1) : B * (A + 1); }
+	__host__ __device__ static constexpr int pad_line() { return A * (B | 1) > B * (A | 1) ? A * (B | 1) : B * (A | 1); }
 	template <int A, int B>
-	__device__ __forceinline__ static int s_pad(int line, int k1, int j) { return line * pad_line<A, B>() + k1 * (B + 1) + j; }
+	__device__ __forceinline__ static int s_pad(int line, int k1, int j) { return line * pad_line<A, B>() + k1 * (B | 1) + j; }
 	template <int A, int B>
 	static constexpr int sm_pad() { return LINES * pad_line<A, B>(); }
 	// split 2 exchanges S(line, a, b), a < A, b < B, rows padded to B+2: the
@@ -152,43 +163,53 @@ __device__ __forceinline__ void line_sync()
 }
 
 // twiddle by table value w = exp(-2 pi i k / N) (conjugated for the inverse)
-template <bool INV>
-__device__ __forceinline__ float2 tw_mul(float2 v, float2 w) { return INV ? cmulc(v, w) : cmul(v, w); }
+template <bool INV, class V>
+__device__ __forceinline__ V tw_mul(V v, float2 w) { return INV ? cmulc(v, w) : cmul(v, w); }
 
 // Stage twiddles W_N^(a b), a on the A-point side of a plan and b on the
 // B-point side: from the N-entry table in global memory (read-only path), or
-// from a CTA's shared copy laid out [a][b] with rows padded to B+2.  A 64-bit
-// shared access is served per half warp, whose 16 lanes need distinct bank
-// pairs: reading W^(k1 j) over consecutive j they have them for any row
-// length, and reading W^(n1 q2) over the pairs (n1 < 8, h; q2 = 2m + h) they
-// sit at (B+2) n1 + h + 2m, distinct modulo 16 because B + 2 = 2 mod 16 for
-// B = 8, 16, 32, 64 (with rows of B+1 the lanes (n1, 1) and (n1 + 1, 0)
-// collided, doubling the wavefronts).
+// from a CTA's shared copy laid out [a][b] with rows of ROW.  A 64-bit shared
+// access is served per half warp, whose 16 lanes need distinct bank pairs.
+// Split 2 reads W^(k1 j) over consecutive j and W^(n1 q2) over the pairs
+// (n1 < 8, h; q2 = 2m + h) at ROW n1 + h + 2m: ROW = B + 2 = 2 mod 16 keeps
+// both distinct (with rows of B+1 the lanes (n1, 1) and (n1 + 1, 0) collided).
+// Split 1 reads along either index, so its rows are odd.
 struct TwGlobal {
 	const float2* p;
 	__device__ __forceinline__ float2 operator()(int a, int b) const { return __ldg(p + a * b); }
 };
-template <int B>
+template <int ROW>
 struct TwShared {
 	const float2* s;
-	__device__ __forceinline__ float2 operator()(int a, int b) const { return s[a * (B + 2) + b]; }
+	__device__ __forceinline__ float2 operator()(int a, int b) const { return s[a * ROW + b]; }
 };
-// Fills a shared [A][B+2] twiddle copy from the global table; the caller
+template <class TW>
+struct TwSwapped {   // the same table with its indices exchanged
+	TW t;
+	__device__ __forceinline__ float2 operator()(int a, int b) const { return t(b, a); }
+};
+// Fills a shared [A][ROW] twiddle copy from the global table; the caller
 // places a CTA barrier before its first use.
-template <int A, int B, int NT>
+template <int A, int B, int ROW, int NT>
 __device__ __forceinline__ void fill_tw_shared(float2* tws, const float2* __restrict__ tw, int tid)
 {
-	for (int i = tid; i < A * (B + 2); i += NT) {
-		const int a = i / (B + 2), b = i - a * (B + 2);
+	for (int i = tid; i < A * ROW; i += NT) {
+		const int a = i / ROW, b = i - a * ROW;
 		tws[i] = b < B ? __ldg(tw + a * b) : make_float2(0.f, 0.f);
 	}
 }
+struct NoPrefetch {
+	__device__ __forceinline__ void operator()() const {}
+};
 
 // ---- split 1 -----------------------------------------------------------------
 // in: B threads/line, thread j holds x[j + B m] (m < A)
 // out: A threads/line, thread k1 holds X[k1 + A k2] (k2 < B)
-template <int A, int B, bool INV, class Tile, int RM, class TW>
-__device__ __forceinline__ void fft_s1_fwd(float2 (&v)[RM], float2* sm, const TW& tw, int tid)
+// LAST: no further exchange follows, so the reads need no barrier after them.
+// prefetch() runs once the exchange is read: loads it issues overlap the
+// second DFT.
+template <int A, int B, bool INV, bool LAST, class Tile, class V, int RM, class TW, class PF>
+__device__ __forceinline__ void fft_s1(V (&v)[RM], V* sm, const TW& tw, int tid, const PF& prefetch)
 {
 	int line, j;
 	Tile::template role<B>(tid, line, j);
@@ -205,32 +226,27 @@ __device__ __forceinline__ void fft_s1_fwd(float2 (&v)[RM], float2* sm, const TW
 	// exchanges under a warp barrier
 	constexpr int P = A > B ? A : B;
 	constexpr bool same = A == B || Tile::kWidth >= P;
-	if constexpr (same) line_sync<Tile, P>();
-	else __syncthreads();
+	auto sync = [] {
+		if constexpr (same) line_sync<Tile, P>();
+		else __syncthreads();
+	};
+	sync();
 	Tile::template role<A>(tid, line, j);
-	if (line < Tile::kLines && j < A) {
+	const bool out_role = line < Tile::kLines && j < A;
+	if (out_role) {
 		#pragma unroll
 		for (int jj = 0; jj < B; jj++) v[jj] = sm[Tile::template s_pad<A, B>(line, j, jj)];
-		dft_reg<B, 1, 0, INV>(v);
 	}
-	if constexpr (same) line_sync<Tile, P>();
-	else __syncthreads();
-}
-
-// in: A threads/line, thread k1 holds x[k1 + A k2] (k2 < B)
-// out: B threads/line, thread j holds y[j + B m] (m < A)
-template <int A, int B, bool INV, class Tile, int RM, class TW>
-__device__ __forceinline__ void fft_s1_inv(float2 (&v)[RM], float2* sm, const TW& tw, int tid)
-{
-	// the transpose of fft_s1_fwd: per-thread B-point DFT, exchange, A-point DFT
-	fft_s1_fwd<B, A, INV, Tile>(v, sm, tw, tid);
+	if constexpr (!LAST) sync();
+	prefetch();
+	if (out_role) dft_reg<B, 1, 0, INV>(v);
 }
 
 // ---- split 2 (B = 2A) ------------------------------------------------------------
 // in: B threads/line, thread j holds x[j + B m] (m < A)
 // out: B threads/line, thread (k1, h) = 2 k1 + h holds X[k1 + A (k + A h)] (k < A)
-template <int A, bool INV, class Tile, int RM, class TW>
-__device__ __forceinline__ void fft_s2_fwd(float2 (&v)[RM], float2* sm, const TW& tw, int tid)
+template <int A, bool INV, class Tile, class V, int RM, class TW, class PF>
+__device__ __forceinline__ void fft_s2_fwd(V (&v)[RM], V* sm, const TW& tw, int tid, const PF& prefetch)
 {
 	constexpr int B = 2 * A;
 	int line, j;
@@ -244,6 +260,8 @@ __device__ __forceinline__ void fft_s2_fwd(float2 (&v)[RM], float2* sm, const TW
 	const int k1 = j >> 1, h = j & 1;
 	#pragma unroll
 	for (int i = 0; i < A; i++) v[i] = sm[Tile::template s_fwd<A, B>(line, k1, 2 * i + h)];
+	line_sync<Tile, B>();
+	prefetch();
 	dft_reg<A, 1, 0, INV>(v);
 	// radix-2 across the pair: Y[k] = E[k] + W_B^k O[k], Y[k + A] = E[k] - W_B^k O[k].
 	// The odd thread twiddles its own value before the exchange, so both
@@ -251,19 +269,15 @@ __device__ __forceinline__ void fft_s2_fwd(float2 (&v)[RM], float2* sm, const TW
 	const float sgn = h ? -1.f : 1.f;
 	static_for<A>([&](auto K) {
 		constexpr int k = K.value;
-		const float2 u = h ? twiddle_ct<k, B, INV>(v[k]) : v[k];
-		float2 o;
-		o.x = __shfl_xor_sync(0xffffffffu, u.x, Tile::kPartner);
-		o.y = __shfl_xor_sync(0xffffffffu, u.y, Tile::kPartner);
-		v[k] = __ffma2_rn(make_float2(sgn, sgn), u, o);
+		const V u = h ? twiddle_ct<k, B, INV>(v[k]) : v[k];
+		v[k] = cfma(sgn, u, cshfl_xor(u, Tile::kPartner));
 	});
-	line_sync<Tile, B>();
 }
 
 // in: B threads/line, thread (n1, h) = 2 n1 + h holds x[n1 + A (k + A h)] (k < A)
 // out: B threads/line, thread j holds y[j + B m] (m < A)
-template <int A, bool INV, class Tile, int RM, class TW>
-__device__ __forceinline__ void fft_s2_inv(float2 (&v)[RM], float2* sm, const TW& tw, int tid)
+template <int A, bool INV, class Tile, class V, int RM, class TW>
+__device__ __forceinline__ void fft_s2_inv(V (&v)[RM], V* sm, const TW& tw, int tid)
 {
 	constexpr int B = 2 * A;
 	int line, j;
@@ -274,10 +288,7 @@ __device__ __forceinline__ void fft_s2_inv(float2 (&v)[RM], float2* sm, const TW
 	const float sgn = h ? -1.f : 1.f;
 	static_for<A>([&](auto K) {
 		constexpr int k = K.value;
-		float2 o;
-		o.x = __shfl_xor_sync(0xffffffffu, v[k].x, Tile::kPartner);
-		o.y = __shfl_xor_sync(0xffffffffu, v[k].y, Tile::kPartner);
-		const float2 d = __ffma2_rn(make_float2(sgn, sgn), v[k], o);
+		const V d = cfma(sgn, v[k], cshfl_xor(v[k], Tile::kPartner));
 		v[k] = h ? twiddle_ct<k, B, INV>(d) : d;
 	});
 	dft_reg<A, 1, 0, INV>(v);   // output q2 = 2 m + h
@@ -291,7 +302,6 @@ __device__ __forceinline__ void fft_s2_inv(float2 (&v)[RM], float2* sm, const TW
 	#pragma unroll
 	for (int i = 0; i < A; i++) v[i] = sm[Tile::template s_inv<A, B>(line, j, i)];
 	dft_reg<A, 1, 0, INV>(v);
-	line_sync<Tile, B>();
 }
 
 // ---- 3 stages, N = R^3 ---------------------------------------------------------
@@ -302,8 +312,8 @@ __device__ __forceinline__ void fft_s2_inv(float2 (&v)[RM], float2* sm, const TW
 //            DFT over m', twiddle W_N^(R j k2), exchange S2;
 //   stage C: thread (k1, k2 = t / R) takes the R values over j, R-point DFT.
 // S1 and S2 are separate regions, so two barriers per transform suffice.
-template <int R, bool INV, class Tile, int RM, class TW>
-__device__ __forceinline__ void fft3(float2 (&v)[RM], float2* sm, const TW& tw, int tid)
+template <int R, bool INV, class Tile, class V, int RM, class TW>
+__device__ __forceinline__ void fft3(V (&v)[RM], V* sm, const TW& tw, int tid)
 {
 	constexpr int T = R * R;
 	int line, t;
@@ -339,27 +349,28 @@ struct Plan {
 	static constexpr int EMID = (S == 2) ? A_ : B_;                    // values per thread (middle layout)
 	static constexpr int TMAX = (T > TMID) ? T : TMID;
 	static constexpr int CC = CC_;                                     // columns per column-pass CTA
-	// the passes keep a shared [A][B+2] copy of the stage twiddles (split 2,
-	// and split 1 with A = B, whose inverse indexes the table the same way)
-	static constexpr bool SMEM_TW = (S == 2 || A_ == B_);
-	static constexpr int TWS = SMEM_TW ? A_ * (B_ + 2) : 1;
+	// the passes keep a shared [A][ROW] copy of the stage twiddles
+	static constexpr bool SMEM_TW = true;
+	static constexpr int ROW = S == 2 ? B_ + 2 : (B_ | 1);
+	static constexpr int TWS = A_ * ROW;
 	// line index of the e-th middle value of position pos
 	__device__ __forceinline__ static int mid(int pos, int e)
 	{
 		if constexpr (S == 2) return (pos >> 1) + A * (e + A * (pos & 1));
 		else return pos + A * e;
 	}
-	template <bool INV, class Tile, class TW>
-	__device__ __forceinline__ static void to_mid(float2 (&v)[RM], float2* sm, const TW& tw, int tid)
+	template <bool INV, class Tile, class V, class TW, class PF = NoPrefetch>
+	__device__ __forceinline__ static void to_mid(V (&v)[RM], V* sm, const TW& tw, int tid, const PF& prefetch = PF{})
 	{
-		if constexpr (S == 2) fft_s2_fwd<A, INV, Tile>(v, sm, tw, tid);
-		else fft_s1_fwd<A, B, INV, Tile>(v, sm, tw, tid);
+		if constexpr (S == 2) fft_s2_fwd<A, INV, Tile>(v, sm, tw, tid, prefetch);
+		else fft_s1<A, B, INV, false, Tile>(v, sm, tw, tid, prefetch);
 	}
-	template <bool INV, class Tile, class TW>
-	__device__ __forceinline__ static void from_mid(float2 (&v)[RM], float2* sm, const TW& tw, int tid)
+	// the last exchange of a pass
+	template <bool INV, class Tile, class V, class TW>
+	__device__ __forceinline__ static void from_mid(V (&v)[RM], V* sm, const TW& tw, int tid)
 	{
 		if constexpr (S == 2) fft_s2_inv<A, INV, Tile>(v, sm, tw, tid);
-		else fft_s1_inv<A, B, INV, Tile>(v, sm, tw, tid);
+		else fft_s1<B, A, INV, true, Tile>(v, sm, TwSwapped<TW>{tw}, tid, NoPrefetch{});
 	}
 	// Threads per line of the row tile in every role: a split-1 plan with
 	// B > A gives its middle role (A threads) the load role's B threads, A of
@@ -396,15 +407,16 @@ struct Plan3 {
 	static constexpr int CC = CC_;
 	static constexpr int ROWW = 0;
 	static constexpr bool SMEM_TW = false;
-	static constexpr int TWS = 1;
+	static constexpr int TWS = 1, ROW = 1;
 	__device__ __forceinline__ static int mid(int pos, int e) { return pos + B * e; }
-	template <bool INV, class Tile, class TW>
-	__device__ __forceinline__ static void to_mid(float2 (&v)[RM], float2* sm, const TW& tw, int tid)
+	template <bool INV, class Tile, class V, class TW, class PF = NoPrefetch>
+	__device__ __forceinline__ static void to_mid(V (&v)[RM], V* sm, const TW& tw, int tid, const PF& prefetch = PF{})
 	{
 		fft3<R_, INV, Tile>(v, sm, tw, tid);
+		prefetch();
 	}
-	template <bool INV, class Tile, class TW>
-	__device__ __forceinline__ static void from_mid(float2 (&v)[RM], float2* sm, const TW& tw, int tid)
+	template <bool INV, class Tile, class V, class TW>
+	__device__ __forceinline__ static void from_mid(V (&v)[RM], V* sm, const TW& tw, int tid)
 	{
 		// the second transform writes S1 before its first barrier; the barriers
 		// of the first transform already ordered all reads of S1 before it
@@ -431,35 +443,55 @@ template <class PL>
 using RowTileOf = RowTile<row_lines<PL>(), PL::ROWW>;
 
 // ---------------------------------------------------------------------------
+// one wave or two waves per element
+// ---------------------------------------------------------------------------
+// A pass runs on single waves (V = float2, work buffer [nwave][ny][nx]) or on
+// pairs of consecutive waves (V = cpair, work buffer [ceil(nwave / 2)][ny][nx]
+// of cpair; with an odd count the last pair's second place repeats its first
+// wave and is not read out).
+template <class V> struct Waves;
+template <> struct Waves<float2> { static constexpr int kN = 1; };
+template <> struct Waves<cpair> { static constexpr int kN = 2; };
+
+template <class V> __device__ __forceinline__ V join(float2 a, float2 b);
+template <> __device__ __forceinline__ float2 join<float2>(float2 a, float2) { return a; }
+template <> __device__ __forceinline__ cpair join<cpair>(float2 a, float2 b)
+{
+	return {make_float2(a.x, b.x), make_float2(a.y, b.y)};
+}
+__device__ __forceinline__ float2 load_v(const float2* p) { return *p; }
+__device__ __forceinline__ cpair load_v(const cpair* p)
+{
+	const float4 q = *reinterpret_cast<const float4*>(p);
+	return {make_float2(q.x, q.y), make_float2(q.z, q.w)};
+}
+__device__ __forceinline__ void store_v(float2* p, float2 v) { *p = v; }
+__device__ __forceinline__ void store_v(cpair* p, cpair v)
+{
+	*reinterpret_cast<float4*>(p) = make_float4(v.re.x, v.re.y, v.im.x, v.im.y);
+}
+// the exchange buffer of a pass
+template <class V>
+__device__ __forceinline__ V* pass_smem()
+{
+	extern __shared__ float4 sm_pass[];
+	return reinterpret_cast<V*>(sm_pass);
+}
+
+// ---------------------------------------------------------------------------
 // readouts
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ float warp_sum(float v)
+// Detector sums: a thread adds its elements of a row in FP32, everything beyond
+// is added in FP64, so the result does not depend on how rows and lanes are
+// grouped (to 1e-16).
+__device__ __forceinline__ double warp_sum(double v)
 {
 	#pragma unroll
 	for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
 	return v;
 }
-
-// Sums acc[d] over the CTA and stores one partial per detector.
-template <int NT>
-__device__ __forceinline__ void block_store_partials(const float (&acc)[kMaxDet], const PassArgs& p, int b)
-{
-	__shared__ float red[NT / 32][kMaxDet];
-	const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-	#pragma unroll
-	for (int d = 0; d < kMaxDet; d++) {
-		float s = warp_sum(acc[d]);
-		if (lane == 0) red[warp][d] = s;
-	}
-	__syncthreads();
-	if ((int)threadIdx.x < p.ndet) {
-		float s = 0.f;
-		#pragma unroll
-		for (int w = 0; w < NT / 32; w++) s += red[w][threadIdx.x];
-		p.partial[(((long long)b * p.ndetslc + p.plane) * p.ndet + threadIdx.x) * p.nblk + blockIdx.x] = s;
-	}
-	__syncthreads();
-}
+__device__ __forceinline__ float fma_w(float pw, float w, float s) { return fmaf(pw, w, s); }
+__device__ __forceinline__ float2 fma_w(float2 pw, float w, float2 s) { return __ffma2_rn(pw, bcast(w), s); }
 
 // Scrambled pixel index at which psi(ky = y, kx) is read out, after the
 // integer-pixel diffraction descan (DescanDifN, src/JMultiSlice.cpp:2184-2273:
@@ -472,60 +504,141 @@ __device__ __forceinline__ void readout_pixel(const PassArgs& p, int& y, int& kx
 	}
 }
 
-// Fourier-space readout of one element psi(ky = y, kx) of wave b
-// (ReadoutDifDet_d, src/JMultiSlice.cpp:4277-4359) except the integrating
-// detectors: diffraction and wave channels, binned pattern.
-__device__ __forceinline__ void readout_fourier_channels(const PassArgs& p, int b, int y, int kx, float2 v)
+// Adds w * f(e), e < E, to the elements idx(e) of a channel: all loads, then all
+// stores (one element after the other, each load would wait for the store
+// before it).
+template <int E, class F, class IX>
+__device__ __forceinline__ void add_channel(float* ch, float w, const F& f, const IX& idx)
 {
-	const long long N = (long long)p.nx * p.ny;
+	float old[E];
+	#pragma unroll
+	for (int e = 0; e < E; e++) old[e] = ch[idx(e)];
+	#pragma unroll
+	for (int e = 0; e < E; e++) ch[idx(e)] = old[e] + w * f(e);
+}
+template <int E, class F, class IX>
+__device__ __forceinline__ void add_channel(float2* ch, float w, const F& f, const IX& idx)
+{
+	float2 old[E];
+	#pragma unroll
+	for (int e = 0; e < E; e++) old[e] = ch[idx(e)];
+	#pragma unroll
+	for (int e = 0; e < E; e++) ch[idx(e)] = __ffma2_rn(f(e), make_float2(w, w), old[e]);
+}
+
+// Adds weight * pw of pixel (y, kx) to the binned pattern of wave b's position.
+__device__ __forceinline__ void readout_bin(const PassArgs& p, int b, int y, int kx, float pw)
+{
 	readout_pixel(p, y, kx);
-	const int idx = y * p.nx + kx;                    // nx * ny < 2^31
-	const float pw = cnorm(v);
-	const long long c = (long long)b * p.chan_wstride + (long long)p.plane * N + idx;
-	if (p.dif) p.dif[c] += p.weight * pw;
-	if (p.dif_avg) p.dif_avg[c] += p.weight * pw;
-	if (p.wff) p.wff[c] = __ffma2_rn(v, make_float2(p.weight, p.weight), p.wff[c]);
-	if (p.wff_avg) p.wff_avg[c] = __ffma2_rn(v, make_float2(p.weight, p.weight), p.wff_avg[c]);
-	if (p.bin_out && p.plane == p.bin_plane) {
-		// unscrambled position (zero beam at nx/2, ny/2 as GetUnscrambleHash,
-		// src/JMultiSlice.cpp:1932-1958), then bin x bin pixel blocks
-		int ux = kx + (p.nx >> 1); if (ux >= p.nx) ux -= p.nx;
-		int uy = y + (p.ny >> 1); if (uy >= p.ny) uy -= p.ny;
-		int bx = ux / p.bin, by = uy / p.bin;
-		const int bp = p.wave_pos > 0 ? b % p.wave_pos : b;   // the wave's probe position
-		if (bx < p.nbx && by < p.nby)
-			atomicAdd(p.bin_out + ((long long)bp * p.nby + by) * p.nbx + bx, p.weight * pw);
+	// unscrambled position (zero beam at nx/2, ny/2 as GetUnscrambleHash,
+	// src/JMultiSlice.cpp:1932-1958), then bin x bin pixel blocks
+	int ux = kx + (p.nx >> 1); if (ux >= p.nx) ux -= p.nx;
+	int uy = y + (p.ny >> 1); if (uy >= p.ny) uy -= p.ny;
+	int bx = ux / p.bin, by = uy / p.bin;
+	const int bp = p.wave_pos > 0 ? b % p.wave_pos : b;   // the wave's probe position
+	if (bx < p.nbx && by < p.nby)
+		atomicAdd(p.bin_out + ((long long)bp * p.nby + by) * p.nbx + bx, p.weight * pw);
+}
+
+// Fourier-space readout of a row tile: thread (y, live) holds the E values v of
+// row y at columns kx_of(e); b0 is the (first) wave.  Called by every thread
+// of the CTA.
+template <int NT, int E, class V, int RM, class KX>
+__device__ __forceinline__ void readout_rows(const PassArgs& p, int b0, int y, bool live, const V (&v)[RM], const KX& kx_of)
+{
+	constexpr int NW = Waves<V>::kN;
+	// channels in loops of their own (uniform tests), so their registers do
+	// not add to those of the other loads
+	if constexpr (NW == 1) {
+		if ((p.dif || p.dif_avg || p.wff || p.wff_avg) && live) {
+			// diffraction and wave channels (ReadoutDifDet_d, src/JMultiSlice.cpp:4277-4359)
+			const long long c = (long long)b0 * p.chan_wstride + (long long)p.plane * p.nx * p.ny;
+			auto idx = [&](int e) {
+				int yd = y, kx = kx_of(e);
+				readout_pixel(p, yd, kx);
+				return yd * p.nx + kx;
+			};
+			auto pw = [&](int e) { return cnorm(v[e]); };
+			auto psi = [&](int e) { return v[e]; };
+			if (p.dif) add_channel<E>(p.dif + c, p.weight, pw, idx);
+			if (p.dif_avg) add_channel<E>(p.dif_avg + c, p.weight, pw, idx);
+			if (p.wff) add_channel<E>(p.wff + c, p.weight, psi, idx);
+			if (p.wff_avg) add_channel<E>(p.wff_avg + c, p.weight, psi, idx);
+		}
+	}
+	const bool two = NW == 2 && b0 + 1 < p.nwave;
+	if (p.bin_out && p.plane == p.bin_plane && live) {
+		#pragma unroll
+		for (int e = 0; e < E; e++) {
+			if constexpr (NW == 1) readout_bin(p, b0, y, kx_of(e), cnorm(v[e]));
+			else {
+				const float2 pw = cnorm(v[e]);
+				readout_bin(p, b0, y, kx_of(e), pw.x);
+				if (two) readout_bin(p, b0 + 1, y, kx_of(e), pw.y);
+			}
+		}
+	}
+	// integrating detectors one at a time (a rolled loop): unrolled over the
+	// detectors, the compiler kept every element's detector loads in flight
+	// (128 registers, half the plain pass's occupancy).  Each warp's sums wait
+	// in shared memory for one CTA barrier after the last detector.
+	__shared__ double red[NT / 32][kMaxDet * NW];
+	const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+	#pragma unroll 1
+	for (int d = 0; d < p.ndet; d++) {
+		const float* det = p.det + (long long)d * p.nx * p.ny;   // detector d: [ny][nx]
+		if constexpr (NW == 1) {
+			float s = 0.f;
+			if (live) {
+				#pragma unroll
+				for (int e = 0; e < E; e++) {
+					int yd = y, kx = kx_of(e);
+					readout_pixel(p, yd, kx);
+					s = fma_w(cnorm(v[e]), __ldg(det + yd * p.nx + kx), s);
+				}
+			}
+			const double t = warp_sum((double)s);
+			if (lane == 0) red[warp][d] = t;
+		}
+		else {
+			float2 s = make_float2(0.f, 0.f);
+			if (live) {
+				#pragma unroll
+				for (int e = 0; e < E; e++) {
+					int yd = y, kx = kx_of(e);
+					readout_pixel(p, yd, kx);
+					s = fma_w(cnorm(v[e]), __ldg(det + yd * p.nx + kx), s);
+				}
+			}
+			const double t0 = warp_sum((double)s.x), t1 = warp_sum((double)s.y);
+			if (lane == 0) { red[warp][2 * d] = t0; red[warp][2 * d + 1] = t1; }
+		}
+	}
+	if (p.ndet > 0) {
+		__syncthreads();
+		const int d = threadIdx.x / NW, w = threadIdx.x % NW;
+		if (d < p.ndet && (w == 0 || two)) {
+			double t = 0.0;
+			#pragma unroll
+			for (int k = 0; k < NT / 32; k++) t += red[k][threadIdx.x];
+			p.partial[(((long long)(b0 + w) * p.ndetslc + p.plane) * p.ndet + d) * p.nblk + blockIdx.x] = t;
+		}
 	}
 }
 
-// Fourier-space readout of one element psi(ky = y, kx) of wave b
-// (ReadoutDifDet_d, src/JMultiSlice.cpp:4277-4359): integrating detectors
-// into acc, then the channels.
-__device__ __forceinline__ void readout_fourier(const PassArgs& p, int b, int y, int kx, float2 v,
-	float (&acc)[kMaxDet])
+// Real-space readout of the E values v of column x at rows y_of(e) of wave b
+// (ReadoutImgDet_d, src/JMultiSlice.cpp:4392-4459).
+template <int E, int RM, class YY>
+__device__ __forceinline__ void readout_cols(const PassArgs& p, int b, int x, const float2 (&v)[RM], const YY& y_of)
 {
-	int yd = y, kxd = kx;
-	readout_pixel(p, yd, kxd);
-	const int idx = yd * p.nx + kxd;                  // nx * ny < 2^31
-	const float pw = cnorm(v);
-	const float* det = p.det + idx;
-	const int N = p.nx * p.ny;
-	#pragma unroll
-	for (int d = 0; d < kMaxDet; d++)
-		if (d < p.ndet) acc[d] = fmaf(pw, __ldg(det + d * N), acc[d]);
-	readout_fourier_channels(p, b, y, kx, v);
-}
-
-// Real-space readout of psi(y, x) of wave b (ReadoutImgDet_d, src/JMultiSlice.cpp:4392-4459).
-__device__ __forceinline__ void readout_real(const PassArgs& p, int b, int y, int x, float2 v)
-{
-	const long long N = (long long)p.nx * p.ny;
-	const long long c = (long long)b * p.chan_wstride + (long long)p.plane * N + (long long)y * p.nx + x;
-	const float pw = cnorm(v);
-	if (p.img) p.img[c] += p.weight * pw;
-	if (p.img_avg) p.img_avg[c] += p.weight * pw;
-	if (p.wfr) p.wfr[c] = __ffma2_rn(v, make_float2(p.weight, p.weight), p.wfr[c]);
-	if (p.wfr_avg) p.wfr_avg[c] = __ffma2_rn(v, make_float2(p.weight, p.weight), p.wfr_avg[c]);
+	const long long c = (long long)b * p.chan_wstride + (long long)p.plane * p.nx * p.ny + x;
+	auto idx = [&](int e) { return y_of(e) * p.nx; };
+	auto pw = [&](int e) { return cnorm(v[e]); };
+	auto psi = [&](int e) { return v[e]; };
+	if (p.img) add_channel<E>(p.img + c, p.weight, pw, idx);
+	if (p.img_avg) add_channel<E>(p.img_avg + c, p.weight, pw, idx);
+	if (p.wfr) add_channel<E>(p.wfr + c, p.weight, psi, idx);
+	if (p.wfr_avg) add_channel<E>(p.wfr_avg + c, p.weight, psi, idx);
 }
 
 // offset phase plate exp(-i (2 pi turns + cppl)) at scrambled pixel (i, j);
@@ -549,67 +662,71 @@ __device__ __forceinline__ float2 offset_factor(const double* sh, int i, int j, 
 	return make_float2(c, -s);
 }
 
+// Element kx of row y of wave b at the entry: the incident wave with the probe
+// offset (phase only where the probe is nonzero, inside its aperture), the wave
+// at wav0, or the work buffer's.
+template <int N>
+__device__ __forceinline__ float2 entry_source(const PassArgs& p, int b, int y, int kx)
+{
+	if (p.shift) {
+		int sx = kx, sy = y;
+		if (p.ibtx | p.ibty) {   // beam tilt: a periodic shift of the incident wave (uniform branch)
+			sx -= p.ibtx; sx %= N; if (sx < 0) sx += N;
+			sy -= p.ibty; sy %= p.ny; if (sy < 0) sy += p.ny;
+		}
+		const float2 a = __ldg(p.wav0 + (long long)sy * N + sx);
+		if (a.x == 0.f && a.y == 0.f) return a;
+		const float cp = p.cppl ? __ldg(p.cppl + (long long)y * N + kx) : 0.f;
+		return cmul(a, offset_factor(p.shift + 4 * b, kx, y, N, p.ny, cp));
+	}
+	return p.wav0 ? __ldg(p.wav0 + (long long)y * N + kx) : p.work[(long long)b * p.wstride + (long long)y * N + kx];
+}
+
 // ---------------------------------------------------------------------------
-// pass kernels (template parameter: the line plan of the transformed axis)
+// pass kernels (template parameters: the line plan of the transformed axis and
+// the element type V)
 // ---------------------------------------------------------------------------
 // Entry row pass: [offset] -> Fourier readout (plane) -> IFT_x.
-template <class PL>
+template <class PL, class V>
 __global__ void __launch_bounds__(row_lines<PL>() * PL::TMAX)
 k_entry_rows(const PassArgs p)
 {
-	constexpr int N = PL::N, L = row_lines<PL>(), NT = L * PL::TMAX;
+	constexpr int N = PL::N, L = row_lines<PL>(), NT = L * PL::TMAX, NW = Waves<V>::kN;
 	using T = RowTileOf<PL>;
-	extern __shared__ float2 sm[];
-	const int tid = threadIdx.x, b = blockIdx.y, row0 = blockIdx.x * L;
+	V* sm = pass_smem<V>();
+	const int tid = threadIdx.x, b = blockIdx.y * NW, row0 = blockIdx.x * L;
+	const int b1 = min(b + 1, p.nwave - 1);
 	const int nval = min(L, p.ny - row0);
 	// Rows outside the source's band of live rows (row_k1 / row_k2: the
 	// incident wave's all-zero rows, for scans without beam tilt) are zero: a
 	// CTA of such rows does nothing, and they are neither read, read out nor
 	// stored (the first column pass reads them as zero).
 	if (row0 > p.row_k1 && row0 + nval - 1 < p.row_k2) return;
-	float2* W = p.work + (long long)b * p.wstride;
-	float2 v[PL::RM];
+	V* W = reinterpret_cast<V*>(p.work) + (long long)blockIdx.y * p.wstride;
+	V v[PL::RM];
 	#pragma unroll
-	for (int m = 0; m < PL::RM; m++) v[m] = make_float2(0.f, 0.f);
-	float acc[kMaxDet];
-	#pragma unroll
-	for (int d = 0; d < kMaxDet; d++) acc[d] = 0.f;
+	for (int m = 0; m < PL::RM; m++) v[m] = czero<V>();
 	int line, j;
 	T::template role<PL::T>(tid, line, j);
-	if (line < nval && (row0 + line <= p.row_k1 || row0 + line >= p.row_k2)) {
-		const int y = row0 + line;
+	const bool live = line < nval && j < PL::T && (row0 + line <= p.row_k1 || row0 + line >= p.row_k2);
+	const int y = row0 + line;
+	if (live) {
 		#pragma unroll
 		for (int m = 0; m < PL::A; m++) {
 			const int kx = j + PL::B * m;
-			float2 a;
-			if (p.shift) {
-				int sx = kx, sy = y;
-				if (p.ibtx | p.ibty) {   // beam tilt: a periodic shift of the incident wave (uniform branch)
-					sx -= p.ibtx; sx %= N; if (sx < 0) sx += N;
-					sy -= p.ibty; sy %= p.ny; if (sy < 0) sy += p.ny;
-				}
-				a = __ldg(p.wav0 + (long long)sy * N + sx);
-				// the offset phase only where the probe is nonzero (inside its aperture)
-				if (a.x != 0.f || a.y != 0.f) {
-					const float cp = p.cppl ? __ldg(p.cppl + (long long)y * N + kx) : 0.f;
-					a = cmul(a, offset_factor(p.shift + 4 * b, kx, y, N, p.ny, cp));
-				}
-			}
-			else {
-				a = p.wav0 ? __ldg(p.wav0 + (long long)y * N + kx) : W[(long long)y * N + kx];
-			}
-			if (p.plane >= 0) readout_fourier(p, b, y, kx, a, acc);
-			v[m] = a;
+			if constexpr (NW == 1) v[m] = entry_source<N>(p, b, y, kx);
+			else if (p.shift || p.wav0) v[m] = join<V>(entry_source<N>(p, b, y, kx), entry_source<N>(p, b1, y, kx));
+			else v[m] = load_v(W + (long long)y * N + kx);
 		}
 	}
-	if (p.plane >= 0 && p.ndet > 0) block_store_partials<NT>(acc, p, b);
+	if (p.plane >= 0) readout_rows<NT, PL::A>(p, b, y, live, v, [&](int m) { return j + PL::B * m; });
 	PL::template to_mid<true, T>(v, sm, TwGlobal{p.twx}, tid);
 	int pos;
 	T::template role<PL::TMID>(tid, line, pos);
 	if (line < nval && pos < PL::TMID && (row0 + line <= p.row_k1 || row0 + line >= p.row_k2)) {
-		float2* dst = W + (long long)(row0 + line) * N;
+		V* dst = W + (long long)(row0 + line) * N;
 		#pragma unroll
-		for (int e = 0; e < PL::EMID; e++) dst[PL::mid(pos, e)] = v[e];
+		for (int e = 0; e < PL::EMID; e++) store_v(dst + PL::mid(pos, e), v[e]);
 	}
 }
 
@@ -617,13 +734,13 @@ k_entry_rows(const PassArgs p)
 // the variant with the readout code (used at readout planes only, as the
 // kernel k_row_pass_read with launch bounds of its own), so the steps without
 // readout do not carry its registers.
-template <class PL, bool READ>
+template <class PL, bool READ, class V>
 __device__ __forceinline__ void row_pass_body(const PassArgs& p)
 {
 	constexpr int N = PL::N, L = row_lines<PL>(), NT = L * PL::TMAX;
 	using T = RowTileOf<PL>;
-	extern __shared__ float2 sm[];
-	const int tid = threadIdx.x, b = blockIdx.y, row0 = blockIdx.x * L;
+	V* sm = pass_smem<V>();
+	const int tid = threadIdx.x, row0 = blockIdx.x * L;
 	const int nval = min(L, p.ny - row0);
 	// rows outside the propagator's band end up exactly zero: a CTA whose rows
 	// are all outside does nothing, and such rows are neither read nor stored
@@ -631,26 +748,40 @@ __device__ __forceinline__ void row_pass_body(const PassArgs& p)
 	if (row0 > p.row_k1 && row0 + nval - 1 < p.row_k2) return;
 	__shared__ float2 tws[PL::TWS];
 	const auto tw = [&] {
-		if constexpr (PL::SMEM_TW) return TwShared<PL::B>{tws};
+		if constexpr (PL::SMEM_TW) return TwShared<PL::ROW>{tws};
 		else return TwGlobal{p.twx};
 	}();
-	float2* W = p.work + (long long)b * p.wstride;
-	float2 v[PL::RM];
+	V* W = reinterpret_cast<V*>(p.work) + (long long)blockIdx.y * p.wstride;
+	V v[PL::RM];
 	#pragma unroll
-	for (int m = 0; m < PL::RM; m++) v[m] = make_float2(0.f, 0.f);
+	for (int m = 0; m < PL::RM; m++) v[m] = czero<V>();
 	int line, j;
 	T::template role<PL::T>(tid, line, j);
 	const int yl = row0 + line;
-	const bool live = line < nval && (yl <= p.row_k1 || yl >= p.row_k2);
+	const bool live = line < nval && j < PL::T && (yl <= p.row_k1 || yl >= p.row_k2);
+	// a launch of few single waves is a chain of latencies: the propagator is
+	// loaded ahead of the wave (pairs have no registers for it)
+	constexpr bool EARLY = Waves<V>::kN == 1 && !READ && PL::EMID <= 16;
+	float2 w[EARLY ? PL::EMID : 1];
+	if constexpr (EARLY) {
+		int l2, pos;
+		T::template role<PL::TMID>(tid, l2, pos);
+		if (l2 < nval && pos < PL::TMID) {
+			const float2* P = p.mul + (long long)(row0 + l2) * N;
+			#pragma unroll
+			for (int e = 0; e < PL::EMID; e++) w[e] = __ldg(P + PL::mid(pos, e));
+		}
+	}
+	if constexpr (EARLY && PL::SMEM_TW) fill_tw_shared<PL::A, PL::B, PL::ROW, NT>(tws, p.twx, tid);
 	if (live) {
-		const float2* src = W + (long long)yl * N;
+		const V* src = W + (long long)yl * N;
 		#pragma unroll
-		for (int m = 0; m < PL::A; m++) v[m] = src[j + PL::B * m];
+		for (int m = 0; m < PL::A; m++) v[m] = load_v(src + j + PL::B * m);
 	}
 	// the twiddle copy is filled while the row loads are in flight, so the
 	// barrier waits for both latencies at once
 	if constexpr (PL::SMEM_TW) {
-		fill_tw_shared<PL::A, PL::B, NT>(tws, p.twx, tid);
+		if constexpr (!EARLY) fill_tw_shared<PL::A, PL::B, PL::ROW, NT>(tws, p.twx, tid);
 		__syncthreads();
 	}
 	// with warp-local lines and no CTA-wide readout, a warp whose lines are
@@ -666,55 +797,21 @@ __device__ __forceinline__ void row_pass_body(const PassArgs& p)
 		if (mid_live) {
 			const float2* P = p.mul + (long long)y * N;
 			#pragma unroll
-			for (int e = 0; e < PL::EMID; e++) v[e] = cmul(v[e], __ldg(P + PL::mid(pos, e)));
-		}
-		if (READ) {
-			// channels in a loop of their own (uniform test), so their
-			// registers do not add to those of the propagator loads
-			const bool chan = p.dif || p.dif_avg || p.wff || p.wff_avg || (p.bin_out && p.plane == p.bin_plane);
-			if (chan && mid_live) {
-				#pragma unroll
-				for (int e = 0; e < PL::EMID; e++) readout_fourier_channels(p, b, y, PL::mid(pos, e), v[e]);
-			}
-			// integrating detectors one at a time (a rolled loop): unrolled
-			// over the detectors, the compiler kept every element's detector
-			// loads in flight (128 registers, half the plain pass's occupancy).
-			// Each warp's sums wait in shared memory for one CTA barrier after
-			// the last detector; the per-warp and per-CTA summation orders are
-			// those of block_store_partials.
-			__shared__ float red[NT / 32][kMaxDet];
-			const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-			for (int d = 0; d < p.ndet; d++) {
-				float s = 0.f;
-				if (mid_live) {
-					const float* det = p.det + (long long)d * p.nx * p.ny;   // detector d: [ny][nx]
-					#pragma unroll
-					for (int e = 0; e < PL::EMID; e++) {
-						int yd = y, kx = PL::mid(pos, e);
-						readout_pixel(p, yd, kx);
-						s = fmaf(cnorm(v[e]), __ldg(det + yd * p.nx + kx), s);
-					}
-				}
-				s = warp_sum(s);
-				if (lane == 0) red[warp][d] = s;
-			}
-			if (p.ndet > 0) {
-				__syncthreads();
-				if ((int)threadIdx.x < p.ndet) {
-					float t = 0.f;
-					#pragma unroll
-					for (int w = 0; w < NT / 32; w++) t += red[w][threadIdx.x];
-					p.partial[(((long long)b * p.ndetslc + p.plane) * p.ndet + threadIdx.x) * p.nblk + blockIdx.x] = t;
-				}
+			for (int e = 0; e < PL::EMID; e++) {
+				if constexpr (EARLY) v[e] = cmul(v[e], w[e]);
+				else v[e] = cmul(v[e], __ldg(P + PL::mid(pos, e)));
 			}
 		}
+		if constexpr (READ)
+			readout_rows<NT, PL::EMID>(p, blockIdx.y * Waves<V>::kN, y, mid_live, v,
+				[&](int e) { return PL::mid(pos, e); });
 	}
 	if (!p.store) return;
 	PL::template from_mid<true, T>(v, sm, tw, tid);
 	if (live) {
-		float2* dst = W + (long long)yl * N;
+		V* dst = W + (long long)yl * N;
 		#pragma unroll
-		for (int m = 0; m < PL::A; m++) dst[j + PL::B * m] = v[m];
+		for (int m = 0; m < PL::A; m++) store_v(dst + j + PL::B * m, v[m]);
 	}
 }
 
@@ -740,18 +837,27 @@ __host__ __device__ constexpr int pass_min_blocks()
 }
 template <class PL>
 __host__ __device__ constexpr int row_min_blocks() { return pass_min_blocks<PL, row_lines<PL>() * PL::TMAX>(); }
-// plain row pass (READ = false); the readout planes use k_row_pass_read
-template <class PL, bool READ>
-__global__ void __launch_bounds__(row_lines<PL>() * PL::TMAX, row_min_blocks<PL>())
+// resident CTAs asked of a pass over wave pairs: at most 128 registers
+template <int NT>
+__host__ __device__ constexpr int pair_min_blocks() { return 65536 / (NT * 128) > 0 ? 65536 / (NT * 128) : 1; }
+template <class PL, class V>
+__host__ __device__ constexpr int row_blocks_sm(bool read)
+{
+	if (Waves<V>::kN == 2) return pair_min_blocks<row_lines<PL>() * PL::TMAX>();
+	return read ? read_min_blocks<PL>() : PL::RM <= 16 ? 0 : row_min_blocks<PL>();
+}
+// plain row pass; the readout planes use k_row_pass_read
+template <class PL, class V>
+__global__ void __launch_bounds__(row_lines<PL>() * PL::TMAX, row_blocks_sm<PL, V>(false))
 k_row_pass(const PassArgs p)
 {
-	row_pass_body<PL, READ>(p);
+	row_pass_body<PL, false, V>(p);
 }
-template <class PL>
-__global__ void __launch_bounds__(row_lines<PL>() * PL::TMAX, read_min_blocks<PL>())
+template <class PL, class V>
+__global__ void __launch_bounds__(row_lines<PL>() * PL::TMAX, row_blocks_sm<PL, V>(true))
 k_row_pass_read(const PassArgs p)
 {
-	row_pass_body<PL, true>(p);
+	row_pass_body<PL, true, V>(p);
 }
 
 // Live rows of a column-pass thread as a bit mask: bit m is set when row
@@ -768,100 +874,164 @@ __device__ __forceinline__ unsigned live_rows(int j, int k1, int k2)
 	return low | high;
 }
 
+// exp(2 pi i (sx x / nx + sy y / ny)): the real-space ramp of a plasmon shift
+__device__ __forceinline__ float2 plasmon_ramp(int sx, int sy, int x, int y, int nx, int ny)
+{
+	const float tx = (float)(int)(((long long)sx * x) % nx) / (float)nx;
+	const float ty = (float)(int)(((long long)sy * y) % ny) / (float)ny;
+	float sn, cs;
+	sincospif(2.f * (tx + ty), &sn, &cs);
+	return make_float2(cs, sn);
+}
+
+// Columns per column-pass CTA: of single waves the plan's own, of wave pairs
+// half of it, so a CTA holds the same shared memory and half the threads; a
+// narrow tile where a launch would leave SMs idle.
+constexpr int kNarrow = 4, kSMs = 148;
+template <class PL, class V>
+__host__ __device__ constexpr int col_width(bool narrow)
+{
+	return narrow && PL::CC / Waves<V>::kN > kNarrow ? kNarrow : PL::CC / Waves<V>::kN;
+}
+
 // Column pass: IFT_y -> real-space readout (plane) -> x t -> FT_y.  NXC is the
 // row stride when it is known at compile time (square grids, nx = N), so the
 // element offsets of the wave and grating accesses are constants; 0 reads it
 // from the arguments.
-// The pass on one tile (wave b, columns col0 ... col0 + C - 1).  SYNC places a
-// CTA barrier between the wave loads and the first transform (which makes a
-// shared twiddle copy filled just before visible).
-template <class PL, bool READ, int NXC, bool SYNC, class TW>
-__device__ __forceinline__ void col_pass_tile(const PassArgs& p, int b, int col0, const TW& tw, float2* sm)
+// The pass on one tile (grid row blockIdx.y, columns col0 ... col0 + C - 1).
+// SYNC places a CTA barrier between the wave loads and the first transform
+// (which makes a shared twiddle copy filled just before visible).
+// The grating of a plan of at most 16 values a thread is loaded into registers
+// early: for wave pairs before the second DFT, whose arithmetic hides the
+// loads' latency (512^2, 512 waves: 449 -> 424 us), for single waves ahead of
+// everything else; larger plans have no registers to spare.
+template <class PL, class V, int C, bool READ, int NXC, bool SYNC, class TW>
+__device__ __forceinline__ void col_pass_tile(const PassArgs& p, int col0, const TW& tw, V* sm)
 {
-	constexpr int C = PL::CC;
+	constexpr int NW = Waves<V>::kN;
+	constexpr bool EARLY = !READ && PL::EMID <= 16;
+	static_assert(!(READ && NW == 2), "images are read out of single waves only");
 	using T = ColTile<C>;
-	const int tid = threadIdx.x;
+	const int tid = threadIdx.x, b = blockIdx.y * NW;
+	const int b1 = min(b + 1, p.nwave - 1);
 	const int nx = NXC > 0 ? NXC : p.nx;
 	const int nval = min(C, nx - col0);
-	float2* W = p.work + (long long)b * p.wstride + col0;
-	float2 v[PL::RM];
+	V* W = reinterpret_cast<V*>(p.work) + (long long)blockIdx.y * p.wstride + col0;
+	V v[PL::RM];
 	#pragma unroll
-	for (int m = 0; m < PL::RM; m++) v[m] = make_float2(0.f, 0.f);
+	for (int m = 0; m < PL::RM; m++) v[m] = czero<V>();
 	int c, j;
 	T::template role<PL::T>(tid, c, j);
+	// element offsets of the waves' gratings
+	const int o0 = p.mul_w ? __ldg(p.mul_w + b) : 0, o1 = NW == 2 && p.mul_w ? __ldg(p.mul_w + b1) : o0;
+	const bool full = p.npgx == nx && p.npgy == p.ny;   // grating of the grid size
+	const bool early = EARLY && full && o0 == o1;
+	int cm, pos;
+	T::template role<PL::TMID>(tid, cm, pos);
+	const bool mid_live = cm < nval && pos < PL::TMID;
+	const int x = col0 + cm;
+	float2 t[EARLY ? PL::EMID : 1];
+	auto load_t = [&] {
+		if constexpr (EARLY) {
+			if (early && mid_live) {
+				const float2* g = p.mul + o0 + x;
+				#pragma unroll
+				for (int e = 0; e < PL::EMID; e++) t[e] = __ldg(g + PL::mid(pos, e) * nx);
+			}
+		}
+	};
+	if constexpr (NW == 1) load_t();
 	// 32-bit offsets within a wave (nx * ny < 2^31): one base pointer per
 	// thread and a row stride, instead of a 64-bit product per element
 	const int stride = PL::B * nx;
 	if (c < nval && j < PL::T) {
-		const float2* src = W + j * nx + c;
+		const V* src = W + j * nx + c;
 		const unsigned lin = live_rows<PL::A, PL::B>(j, p.in_k1, p.in_k2);
 		#pragma unroll
 		for (int m = 0; m < PL::A; m++)
-			if (lin & (1u << m)) v[m] = src[m * stride];
+			if (lin & (1u << m)) v[m] = load_v(src + m * stride);
 	}
 	if constexpr (SYNC) __syncthreads();
-	PL::template to_mid<true, T>(v, sm, tw, tid);
-	{
-		int pos;
-		T::template role<PL::TMID>(tid, c, pos);
-		if (c < nval && pos < PL::TMID) {
-			const int x = col0 + c;
-			const float2* mul = p.mul + (p.mul_w ? __ldg(p.mul_w + b) : 0);   // this wave's grating
-			if (p.npgx == nx && p.npgy == p.ny) { // grating of the grid size
-				const float2* t = mul + x;
+	PL::template to_mid<true, T>(v, sm, tw, tid, [&] {
+		if constexpr (NW == 2) load_t();
+	});
+	if (mid_live) {
+		if constexpr (READ) readout_cols<PL::EMID>(p, b, x, v, [&](int e) { return PL::mid(pos, e); });
+		const float2* mul = p.mul + o0;
+		if (early) {
+			if constexpr (EARLY) {
 				#pragma unroll
-				for (int e = 0; e < PL::EMID; e++) {
-					const int y = PL::mid(pos, e);
-					if (READ) readout_real(p, b, y, x, v[e]);
-					v[e] = cmul(v[e], __ldg(t + y * nx));
-				}
+				for (int e = 0; e < PL::EMID; e++) v[e] = cmul(v[e], t[e]);
+			}
+		}
+		else if (NW == 1 || o0 == o1) {
+			if (full) {
+				#pragma unroll
+				for (int e = 0; e < PL::EMID; e++) v[e] = cmul(v[e], __ldg(mul + x + PL::mid(pos, e) * nx));
 			}
 			else { // sub-frame grating repeated periodically
 				const int xs = x % p.npgx;
 				#pragma unroll
-				for (int e = 0; e < PL::EMID; e++) {
-					const int y = PL::mid(pos, e);
-					if (READ) readout_real(p, b, y, x, v[e]);
-					v[e] = cmul(v[e], __ldg(mul + (long long)(y % p.npgy) * p.npgx + xs));
-				}
+				for (int e = 0; e < PL::EMID; e++)
+					v[e] = cmul(v[e], __ldg(mul + (long long)(PL::mid(pos, e) % p.npgy) * p.npgx + xs));
 			}
-			int sx = p.plas_x, sy = p.plas_y;
-			if (p.plas_w) { sx = __ldg(p.plas_w + 2 * b); sy = __ldg(p.plas_w + 2 * b + 1); }
-			if (sx | sy) { // plasmon shift of the spectrum (uniform branch)
-				const float tx = (float)(int)(((long long)sx * x) % nx) / (float)nx;
-				#pragma unroll
-				for (int e = 0; e < PL::EMID; e++) {
-					const int y = PL::mid(pos, e);
-					const float ty = (float)(int)(((long long)sy * y) % p.ny) / (float)p.ny;
-					float sn, cs;
-					sincospif(2.f * (tx + ty), &sn, &cs);
-					v[e] = cmul(v[e], make_float2(cs, sn));
-				}
+		}
+		else if constexpr (NW == 2) { // the two waves are of different configurations
+			const float2* mul1 = p.mul + o1;
+			const int xs = full ? x : x % p.npgx;
+			#pragma unroll
+			for (int e = 0; e < PL::EMID; e++) {
+				const int y = PL::mid(pos, e);
+				const int q = (full ? y : y % p.npgy) * p.npgx + xs;
+				v[e] = cmul(v[e], __ldg(mul + q), __ldg(mul1 + q));
+			}
+		}
+		int sx = p.plas_x, sy = p.plas_y, sx1 = 0, sy1 = 0;
+		if (p.plas_w) {
+			sx = __ldg(p.plas_w + 2 * b); sy = __ldg(p.plas_w + 2 * b + 1);
+			if constexpr (NW == 2) { sx1 = __ldg(p.plas_w + 2 * b1); sy1 = __ldg(p.plas_w + 2 * b1 + 1); }
+		}
+		if (sx | sy | sx1 | sy1) { // plasmon shift of the spectrum (uniform branch)
+			#pragma unroll
+			for (int e = 0; e < PL::EMID; e++) {
+				const int y = PL::mid(pos, e);
+				const float2 r = plasmon_ramp(sx, sy, x, y, nx, p.ny);
+				if constexpr (NW == 1) v[e] = cmul(v[e], r);
+				else v[e] = cmul(v[e], r, plasmon_ramp(sx1, sy1, x, y, nx, p.ny));
 			}
 		}
 	}
 	PL::template from_mid<false, T>(v, sm, tw, tid);
 	T::template role<PL::T>(tid, c, j);
 	if (c < nval && j < PL::T) {
-		float2* dst = W + j * nx + c;
+		V* dst = W + j * nx + c;
 		const unsigned lout = live_rows<PL::A, PL::B>(j, p.out_k1, p.out_k2);
 		#pragma unroll
 		for (int m = 0; m < PL::A; m++)
-			if (lout & (1u << m)) dst[m * stride] = v[m];
+			if (lout & (1u << m)) store_v(dst + m * stride, v[m]);
 	}
 }
 
-template <class PL, bool READ, int NXC>
-__global__ void __launch_bounds__(PL::CC * PL::TMAX, PL::RM > 16 && !READ ? pass_min_blocks<PL, PL::CC * PL::TMAX>() : 0)
+// Resident CTAs asked of a column pass: wave pairs at most 128 registers;
+// single waves of the full width as the row pass; narrow tiles are few and free.
+template <class PL, class V, int C>
+__host__ __device__ constexpr int col_blocks_sm(bool read)
+{
+	constexpr int NT = C * PL::TMAX;
+	if (Waves<V>::kN == 2) return pair_min_blocks<NT>();
+	return PL::RM > 16 && !read ? pass_min_blocks<PL, NT>() : 0;
+}
+template <class PL, class V, int C, bool READ, int NXC>
+__global__ void __launch_bounds__(C * PL::TMAX, col_blocks_sm<PL, V, C>(READ))
 k_col_pass(const PassArgs p)
 {
-	extern __shared__ float2 sm[];
+	V* sm = pass_smem<V>();
 	__shared__ float2 tws[PL::TWS];
 	if constexpr (PL::SMEM_TW) {
-		fill_tw_shared<PL::A, PL::B, PL::CC * PL::TMAX>(tws, p.twy, threadIdx.x);   // barrier after the wave loads
-		col_pass_tile<PL, READ, NXC, true>(p, blockIdx.y, blockIdx.x * PL::CC, TwShared<PL::B>{tws}, sm);
+		fill_tw_shared<PL::A, PL::B, PL::ROW, C * PL::TMAX>(tws, p.twy, threadIdx.x);   // barrier after the wave loads
+		col_pass_tile<PL, V, C, READ, NXC, true>(p, blockIdx.x * C, TwShared<PL::ROW>{tws}, sm);
 	}
-	else col_pass_tile<PL, READ, NXC, false>(p, blockIdx.y, blockIdx.x * PL::CC, TwGlobal{p.twy}, sm);
+	else col_pass_tile<PL, V, C, READ, NXC, false>(p, blockIdx.x * C, TwGlobal{p.twy}, sm);
 }
 
 // Exit column pass: IFT_y -> real-space readout (plane), no store.
@@ -871,7 +1041,7 @@ k_exit_cols(const PassArgs p)
 {
 	constexpr int C = PL::CC;
 	using T = ColTile<C>;
-	extern __shared__ float2 sm[];
+	float2* sm = pass_smem<float2>();
 	const int tid = threadIdx.x, b = blockIdx.y, col0 = blockIdx.x * C;
 	const int nval = min(C, p.nx - col0);
 	const int nx = p.nx;
@@ -891,10 +1061,7 @@ k_exit_cols(const PassArgs p)
 	PL::template to_mid<true, T>(v, sm, TwGlobal{p.twy}, tid);
 	int pos;
 	T::template role<PL::TMID>(tid, c, pos);
-	if (c < nval && pos < PL::TMID) {
-		#pragma unroll
-		for (int e = 0; e < PL::EMID; e++) readout_real(p, b, PL::mid(pos, e), col0 + c, v[e]);
-	}
+	if (c < nval && pos < PL::TMID) readout_cols<PL::EMID>(p, b, col0 + c, v, [&](int e) { return PL::mid(pos, e); });
 }
 
 // ---------------------------------------------------------------------------
@@ -908,7 +1075,7 @@ template <class K>
 cudaError_t launch_k(K kern, dim3 grid, int threads, int smem, const PassArgs& p, cudaStream_t s)
 {
 	static_assert(sizeof(PassArgs) < 4000, "kernel parameter block too large");
-	if (smem > 48 * 1024) {
+	if (smem > 16 * 1024) {   // the default limit of 48 KB includes a kernel's static part
 		cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
 		if (e != cudaSuccess) return e;
 	}
@@ -919,34 +1086,46 @@ cudaError_t launch_k(K kern, dim3 grid, int threads, int smem, const PassArgs& p
 template <class PL>
 int row_blocks_t(int ny) { return (ny + row_lines<PL>() - 1) / row_lines<PL>(); }
 
-template <class PL>
+// grid rows: waves, or pairs of waves
+template <class V>
+unsigned wave_rows(const PassArgs& p) { return (unsigned)((p.nwave + Waves<V>::kN - 1) / Waves<V>::kN); }
+
+template <class PL, class V>
 cudaError_t launch_entry_t(const PassArgs& p, cudaStream_t s)
 {
 	constexpr int L = row_lines<PL>();
-	constexpr int smem = PL::template smem_elems<RowTileOf<PL>>() * (int)sizeof(float2);
-	return launch_k(k_entry_rows<PL>, dim3((p.ny + L - 1) / L, p.nwave), L * PL::TMAX, smem, p, s);
+	constexpr int smem = PL::template smem_elems<RowTileOf<PL>>() * (int)sizeof(V);
+	return launch_k(k_entry_rows<PL, V>, dim3((p.ny + L - 1) / L, wave_rows<V>(p)), L * PL::TMAX, smem, p, s);
 }
-template <class PL>
+template <class PL, class V>
 cudaError_t launch_row_t(const PassArgs& p, cudaStream_t s)
 {
 	constexpr int L = row_lines<PL>();
-	constexpr int smem = PL::template smem_elems<RowTileOf<PL>>() * (int)sizeof(float2);
-	const dim3 grid((p.ny + L - 1) / L, p.nwave);
-	if (p.plane >= 0) return launch_k(k_row_pass_read<PL>, grid, L * PL::TMAX, smem, p, s);
-	return launch_k(k_row_pass<PL, false>, grid, L * PL::TMAX, smem, p, s);
+	constexpr int smem = PL::template smem_elems<RowTileOf<PL>>() * (int)sizeof(V);
+	const dim3 grid((p.ny + L - 1) / L, wave_rows<V>(p));
+	if (p.plane >= 0) return launch_k(k_row_pass_read<PL, V>, grid, L * PL::TMAX, smem, p, s);
+	return launch_k(k_row_pass<PL, V>, grid, L * PL::TMAX, smem, p, s);
 }
-template <class PL>
+template <class PL, class V, int C, bool READ, int NXC>
+cudaError_t launch_col_c(const PassArgs& p, cudaStream_t s)
+{
+	constexpr int smem = PL::template smem_elems<ColTile<C>>() * (int)sizeof(V);
+	return launch_k(k_col_pass<PL, V, C, READ, NXC>, dim3((p.nx + C - 1) / C, wave_rows<V>(p)), C * PL::TMAX, smem, p, s);
+}
+template <class PL, class V>
 cudaError_t launch_col_t(const PassArgs& p, cudaStream_t s)
 {
-	constexpr int C = PL::CC;
-	constexpr int smem = PL::template smem_elems<ColTile<C>>() * (int)sizeof(float2);
-	const dim3 grid((p.nx + C - 1) / C, p.nwave);
-	if (p.plane >= 0) {
-		if (p.nx == PL::N) return launch_k(k_col_pass<PL, true, PL::N>, grid, C * PL::TMAX, smem, p, s);
-		return launch_k(k_col_pass<PL, true, 0>, grid, C * PL::TMAX, smem, p, s);
+	constexpr int C = col_width<PL, V>(false), CN = col_width<PL, V>(true);
+	if constexpr (Waves<V>::kN == 1) {
+		if (p.plane >= 0)
+			return p.nx == PL::N ? launch_col_c<PL, V, C, true, PL::N>(p, s) : launch_col_c<PL, V, C, true, 0>(p, s);
+		// fewer tiles than SMs: narrow tiles, for lines long enough to fill
+		// their warps (one wave: 512^2 7.1 -> 5.4 us per launch, 256^2 4.5
+		// either way, 64^2 2.5 -> 3.3)
+		if constexpr (PL::N >= 320)
+			if ((long long)((p.nx + C - 1) / C) * p.nwave < kSMs) return launch_col_c<PL, V, CN, false, 0>(p, s);
 	}
-	if (p.nx == PL::N) return launch_k(k_col_pass<PL, false, PL::N>, grid, C * PL::TMAX, smem, p, s);
-	return launch_k(k_col_pass<PL, false, 0>, grid, C * PL::TMAX, smem, p, s);
+	return p.nx == PL::N ? launch_col_c<PL, V, C, false, PL::N>(p, s) : launch_col_c<PL, V, C, false, 0>(p, s);
 }
 template <class PL>
 cudaError_t launch_exit_t(const PassArgs& p, cudaStream_t s)
@@ -956,11 +1135,21 @@ cudaError_t launch_exit_t(const PassArgs& p, cudaStream_t s)
 	return launch_k(k_exit_cols<PL>, dim3((p.nx + C - 1) / C, p.nwave), C * PL::TMAX, smem, p, s);
 }
 
-#define JMS_INSTANTIATE(PL) \
-	template int row_blocks_t<PL>(int); \
-	template cudaError_t launch_entry_t<PL>(const PassArgs&, cudaStream_t); \
-	template cudaError_t launch_row_t<PL>(const PassArgs&, cudaStream_t); \
-	template cudaError_t launch_col_t<PL>(const PassArgs&, cudaStream_t); \
-	template cudaError_t launch_exit_t<PL>(const PassArgs&, cudaStream_t);
+// The passes of a plan.  Wave pairs need the plan's values twice in registers:
+// plans of at most 16 values a thread have them.
+template <class PL>
+PlanOps plan_ops_t(int n, const char* name)
+{
+	PlanOps o = {n, name, &row_blocks_t<PL>, &launch_entry_t<PL, float2>, &launch_row_t<PL, float2>,
+		&launch_col_t<PL, float2>, &launch_exit_t<PL>, nullptr, nullptr, nullptr};
+	if constexpr (PL::RM <= 16) {
+		o.entry2 = &launch_entry_t<PL, cpair>;
+		o.row2 = &launch_row_t<PL, cpair>;
+		o.col2 = &launch_col_t<PL, cpair>;
+	}
+	return o;
+}
+
+#define JMS_INSTANTIATE(PL) template PlanOps plan_ops_t<PL>(int, const char*);
 
 } // namespace jms

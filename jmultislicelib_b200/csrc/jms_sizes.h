@@ -43,11 +43,7 @@ using P1024b = Plan<32, 32, 8>;
 using P2048a = Plan<32, 64, 8>;
 using P2048b = Plan<32, 64, 4>;
 
-template <class PL> int row_blocks_t(int ny);
-template <class PL> cudaError_t launch_entry_t(const PassArgs& p, cudaStream_t s);
-template <class PL> cudaError_t launch_row_t(const PassArgs& p, cudaStream_t s);
-template <class PL> cudaError_t launch_col_t(const PassArgs& p, cudaStream_t s);
-template <class PL> cudaError_t launch_exit_t(const PassArgs& p, cudaStream_t s);
+template <class PL> PlanOps plan_ops_t(int n, const char* name);
 } // namespace jms
 
 // X(length, plan alias, printable name); the first entry of a length is its default
