@@ -470,6 +470,14 @@ __device__ __forceinline__ void store_v(cpair* p, cpair v)
 {
 	*reinterpret_cast<float4*>(p) = make_float4(v.re.x, v.re.y, v.im.x, v.im.y);
 }
+// Programmatic launches: a pass lets the next one start once all its CTAs run
+// (its twiddles, and single waves' gratings and propagators, are then loaded
+// while this one finishes), and waits for the previous one's results before it
+// touches the waves.  Every CTA waits, also one with nothing to do, so a pass
+// never ends before the one ahead of it.
+__device__ __forceinline__ void pass_trigger() { asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory"); }
+__device__ __forceinline__ void pass_wait() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
+
 // the exchange buffer of a pass
 template <class V>
 __device__ __forceinline__ V* pass_smem()
@@ -745,7 +753,11 @@ __device__ __forceinline__ void row_pass_body(const PassArgs& p)
 	// rows outside the propagator's band end up exactly zero: a CTA whose rows
 	// are all outside does nothing, and such rows are neither read nor stored
 	// (the column pass reads them as zero)
-	if (row0 > p.row_k1 && row0 + nval - 1 < p.row_k2) return;
+	pass_trigger();
+	if (row0 > p.row_k1 && row0 + nval - 1 < p.row_k2) {
+		pass_wait();
+		return;
+	}
 	__shared__ float2 tws[PL::TWS];
 	const auto tw = [&] {
 		if constexpr (PL::SMEM_TW) return TwShared<PL::ROW>{tws};
@@ -760,7 +772,7 @@ __device__ __forceinline__ void row_pass_body(const PassArgs& p)
 	const int yl = row0 + line;
 	const bool live = line < nval && j < PL::T && (yl <= p.row_k1 || yl >= p.row_k2);
 	// a launch of few single waves is a chain of latencies: the propagator is
-	// loaded ahead of the wave (pairs have no registers for it)
+	// loaded ahead of the wait (pairs have no registers for it)
 	constexpr bool EARLY = Waves<V>::kN == 1 && !READ && PL::EMID <= 16;
 	float2 w[EARLY ? PL::EMID : 1];
 	if constexpr (EARLY) {
@@ -773,6 +785,7 @@ __device__ __forceinline__ void row_pass_body(const PassArgs& p)
 		}
 	}
 	if constexpr (EARLY && PL::SMEM_TW) fill_tw_shared<PL::A, PL::B, PL::ROW, NT>(tws, p.twx, tid);
+	pass_wait();
 	if (live) {
 		const V* src = W + (long long)yl * N;
 		#pragma unroll
@@ -940,7 +953,8 @@ __device__ __forceinline__ void col_pass_tile(const PassArgs& p, int col0, const
 			}
 		}
 	};
-	if constexpr (NW == 1) load_t();
+	if constexpr (NW == 1) load_t();   // single waves: ahead of the wait
+	pass_wait();
 	// 32-bit offsets within a wave (nx * ny < 2^31): one base pointer per
 	// thread and a row stride, instead of a 64-bit product per element
 	const int stride = PL::B * nx;
@@ -1025,6 +1039,7 @@ template <class PL, class V, int C, bool READ, int NXC>
 __global__ void __launch_bounds__(C * PL::TMAX, col_blocks_sm<PL, V, C>(READ))
 k_col_pass(const PassArgs p)
 {
+	pass_trigger();
 	V* sm = pass_smem<V>();
 	__shared__ float2 tws[PL::TWS];
 	if constexpr (PL::SMEM_TW) {
@@ -1071,16 +1086,26 @@ k_exit_cols(const PassArgs p)
 // atom chunks with them)
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
 
+// chained: a pass kernel that waits for the one ahead of it itself (pass_wait)
 template <class K>
-cudaError_t launch_k(K kern, dim3 grid, int threads, int smem, const PassArgs& p, cudaStream_t s)
+cudaError_t launch_k(K kern, dim3 grid, int threads, int smem, const PassArgs& p, cudaStream_t s, bool chained = false)
 {
 	static_assert(sizeof(PassArgs) < 4000, "kernel parameter block too large");
 	if (smem > 16 * 1024) {   // the default limit of 48 KB includes a kernel's static part
 		cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
 		if (e != cudaSuccess) return e;
 	}
-	kern<<<grid, threads, smem, s>>>(p);
-	return cudaGetLastError();
+	cudaLaunchConfig_t cfg = {};
+	cfg.gridDim = grid;
+	cfg.blockDim = dim3(threads);
+	cfg.dynamicSmemBytes = smem;
+	cfg.stream = s;
+	cudaLaunchAttribute at;
+	at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+	at.val.programmaticStreamSerializationAllowed = 1;
+	cfg.attrs = &at;
+	cfg.numAttrs = chained ? 1 : 0;
+	return cudaLaunchKernelEx(&cfg, kern, p);
 }
 
 template <class PL>
@@ -1103,14 +1128,15 @@ cudaError_t launch_row_t(const PassArgs& p, cudaStream_t s)
 	constexpr int L = row_lines<PL>();
 	constexpr int smem = PL::template smem_elems<RowTileOf<PL>>() * (int)sizeof(V);
 	const dim3 grid((p.ny + L - 1) / L, wave_rows<V>(p));
-	if (p.plane >= 0) return launch_k(k_row_pass_read<PL, V>, grid, L * PL::TMAX, smem, p, s);
-	return launch_k(k_row_pass<PL, V>, grid, L * PL::TMAX, smem, p, s);
+	if (p.plane >= 0) return launch_k(k_row_pass_read<PL, V>, grid, L * PL::TMAX, smem, p, s, true);
+	return launch_k(k_row_pass<PL, V>, grid, L * PL::TMAX, smem, p, s, true);
 }
 template <class PL, class V, int C, bool READ, int NXC>
 cudaError_t launch_col_c(const PassArgs& p, cudaStream_t s)
 {
 	constexpr int smem = PL::template smem_elems<ColTile<C>>() * (int)sizeof(V);
-	return launch_k(k_col_pass<PL, V, C, READ, NXC>, dim3((p.nx + C - 1) / C, wave_rows<V>(p)), C * PL::TMAX, smem, p, s);
+	return launch_k(k_col_pass<PL, V, C, READ, NXC>, dim3((p.nx + C - 1) / C, wave_rows<V>(p)), C * PL::TMAX, smem, p, s,
+		true);
 }
 template <class PL, class V>
 cudaError_t launch_col_t(const PassArgs& p, cudaStream_t s)
