@@ -1161,10 +1161,14 @@ int JmsB200::ScanGPUDevice(int npos, const float* d_pos, float dz, int npass, co
 	const int B = std::max(1, scan_batch_);
 	std::vector<int> var((size_t)nobjslc_), plas_h;
 	const float w = 1.f / (float)npass;
-	// Fused configurations: with fewer positions than the batch, kp
-	// configurations of all positions share one launch sequence, wave
-	// k * npos + p being position p in configuration k.  Needs no plasmon
-	// paths and grating offsets within int range.
+	// Waves of a launch sequence.  Configurations share launches where a batch
+	// has room for them, and batches of small grids are put together up to
+	// kMergePoints wave points (64 MB, which stays in L2): 32 waves of 128^2 fill
+	// a fifth of the GPU and run at launch latency.  Wave k * np + p is position p
+	// in configuration k.  Needs no plasmon paths and grating offsets within int
+	// range.
+	constexpr long long kMergePoints = 1LL << 23;
+	const int Wm = (int)std::max<long long>(B, kMergePoints / std::max(1LL, (long long)nx_ * ny_));
 	const long long pool = slcoffset_.empty() ? 0
 		: slcoffset_.back() + (long long)nvarslc_.back() * npgx_ * npgy_;
 	// A stream capture keeps the sequential form: the fused form uploads its
@@ -1172,18 +1176,23 @@ int JmsB200::ScanGPUDevice(int npos, const float* d_pos, float dz, int npass, co
 	// replay.
 	cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
 	if (stream_) cudaStreamIsCapturing(stream_, &cap);
-	if (fuse_passes_ && npass > 1 && npos < B && !plasmon_on_ && pool < (1LL << 31) &&
-		cap == cudaStreamCaptureStatusNone) {
-		// without a given sequence, draw every configuration now, in the order
-		// the sequential form would (one draw per pass, positions in one batch)
+	const bool merge = (npass > 1 && npos < B) || (Wm > B && (npass > 1 || npos > B));
+	if (fuse_passes_ && merge && !plasmon_on_ && pool < (1LL << 31) && cap == cudaStreamCaptureStatusNone) {
+		// Without a given sequence, draw every configuration now, in the order
+		// the sequential form would: one draw per batch of positions and pass.
+		const int nbatch = (npos + B - 1) / B;
 		std::vector<int> drawn;
 		if (!varseq) {
-			drawn.resize((size_t)npass * nobjslc_);
-			for (int ip = 0; ip < npass; ip++) GetRandomVariantSequence(drawn.data() + (size_t)ip * nobjslc_);
-			varseq = drawn.data();
+			drawn.resize((size_t)nbatch * npass * nobjslc_);
+			for (int k = 0; k < nbatch * npass; k++) GetRandomVariantSequence(drawn.data() + (size_t)k * nobjslc_);
 		}
-		const int kp = std::min(npass, std::max(1, B / npos));
-		const size_t nw_max = (size_t)kp * npos;
+		// variants of position p in pass ip
+		auto variants = [&](int p, int ip) {
+			return varseq ? varseq + (size_t)ip * nobjslc_ : drawn.data() + ((size_t)(p / B) * npass + ip) * nobjslc_;
+		};
+		const int np_max = std::min(npos, Wm);      // positions per launch
+		const int kp = std::min(npass, std::max(1, Wm / np_max));
+		const size_t nw_max = (size_t)kp * np_max;
 		if (nw_max * 4 > shiftw_cap_) {
 			dfree(d_shiftw_);
 			shiftw_cap_ = 0;
@@ -1197,29 +1206,32 @@ int JmsB200::ScanGPUDevice(int npos, const float* d_pos, float dz, int npass, co
 			if (post(cudaMalloc(&d_mulw_, sizeof(int) * nw_max * nobjslc_), "ScanGPU")) return 1;
 			mulw_cap_ = nw_max * nobjslc_;
 		}
-		for (int ip0 = 0; ip0 < npass; ip0 += kp) {
-			const int kk = std::min(kp, npass - ip0), nw = kk * npos;
-			h_mulw_.assign((size_t)nw * nobjslc_, 0);
-			for (int j = 0; j < nobjslc_; j++) {
-				const int st = objslc_[j] % nscslc_;
-				for (int k = 0; k < kk; k++) {
-					const int v = varseq[(size_t)(ip0 + k) * nobjslc_ + j];
-					const int off = (int)(slcoffset_[st] + (long long)v * npgx_ * npgy_);
-					for (int p = 0; p < npos; p++) h_mulw_[(size_t)j * nw + (size_t)k * npos + p] = off;
-				}
+		for (int p0 = 0; p0 < npos; p0 += np_max)
+			for (int ip0 = 0; ip0 < npass; ip0 += kp) {
+				const int np = std::min(np_max, npos - p0), kk = std::min(kp, npass - ip0), nw = kk * np;
+				h_mulw_.assign((size_t)nw * nobjslc_, 0);
+				for (int k = 0; k < kk; k++)
+					for (int p = 0; p < np; p++) {
+						const int* var = variants(p0 + p, ip0 + k);
+						for (int j = 0; j < nobjslc_; j++) {
+							const int st = objslc_[j] % nscslc_;
+							h_mulw_[(size_t)j * nw + (size_t)k * np + p] =
+								(int)(slcoffset_[st] + (long long)var[j] * npgx_ * npgy_);
+						}
+					}
+				// stream order keeps the previous launch sequence's reads of the
+				// tables ahead of these writes
+				if (post(cudaMemcpyAsync(d_mulw_, h_mulw_.data(), sizeof(int) * h_mulw_.size(), cudaMemcpyHostToDevice,
+					stream_), "ScanGPU")) return 1;
+				if (post(launch_gather_shift(d_shiftw_, d_shift_ + (size_t)p0 * 4, np, nw, stream_), "ScanGPU")) return 1;
+				launches_++;
+				int e = run_slices(nw, 0, nullptr, w, d_wav0_, d_shiftw_, 0, 0, d_cppl_,
+					d_out_int ? d_out_int + (size_t)p0 * ndetslc_ * ndet_ : nullptr,
+					d_out_bin ? d_out_bin + (size_t)p0 * nbx * nby : nullptr, bin, nbx, nby, nullptr, nullptr, d_mulw_, np);
+				if (e) return e;
+				// the pageable host table is reused by the next group: its copy above
+				// has been staged already when cudaMemcpyAsync returned
 			}
-			// stream order keeps the previous launch sequence's reads of the
-			// tables ahead of these writes
-			if (post(cudaMemcpyAsync(d_mulw_, h_mulw_.data(), sizeof(int) * h_mulw_.size(), cudaMemcpyHostToDevice,
-				stream_), "ScanGPU")) return 1;
-			if (post(launch_gather_shift(d_shiftw_, d_shift_, npos, nw, stream_), "ScanGPU")) return 1;
-			launches_++;
-			int e = run_slices(nw, 0, nullptr, w, d_wav0_, d_shiftw_, 0, 0, d_cppl_, d_out_int, d_out_bin, bin, nbx, nby,
-				nullptr, nullptr, d_mulw_, npos);
-			if (e) return e;
-			// the pageable host table is reused by the next group: its copy above
-			// has been staged already when cudaMemcpyAsync returned
-		}
 		return 0;
 	}
 	for (int p0 = 0; p0 < npos; p0 += B) {
