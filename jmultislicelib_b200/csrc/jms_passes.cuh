@@ -69,6 +69,9 @@ struct RowTile {
 	// warp barriers, and the warps of a CTA run their lines independently.
 	template <int P>
 	__host__ __device__ static constexpr bool warp_lines() { return 32 % (W > 0 ? W : P) == 0; }
+	// Lines of two or more whole warps synchronise by themselves (barriers 1 to 15).
+	template <int P>
+	__host__ __device__ static constexpr bool own_barrier() { return W == 0 && P > 32 && P % 32 == 0 && LINES <= 15; }
 	// split 1 exchange S(line, k1, j), k1 < A, j < B, rows of odd length.  A
 	// line's region has the same size for <A, B> and <B, A> (the forward and
 	// inverse exchanges), so with warp-local lines one line's inverse exchange
@@ -130,6 +133,8 @@ struct ColTile {
 	__device__ __forceinline__ static void role(int tid, int& line, int& pos) { line = tid % C; pos = tid / C; }
 	template <int P>
 	__host__ __device__ static constexpr bool warp_lines() { return false; }   // a column's positions span warps
+	template <int P>
+	__host__ __device__ static constexpr bool own_barrier() { return false; }
 	template <int A, int B>
 	__device__ __forceinline__ static int s_pad(int line, int k1, int j) { return k1 * (B * C + PAD) + j * C + line; }
 	template <int A, int B>
@@ -154,11 +159,14 @@ struct ColTile {
 
 // Barrier around an exchange of lines of P threads: a warp barrier (which also
 // orders the warp's shared-memory accesses) when every line and its exchange
-// region lie inside one warp, else a CTA barrier.
+// region lie inside one warp, a named barrier of the line's own where it is a
+// few whole warps, else a CTA barrier.
 template <class Tile, int P>
 __device__ __forceinline__ void line_sync()
 {
 	if constexpr (Tile::template warp_lines<P>()) __syncwarp();
+	else if constexpr (Tile::template own_barrier<P>())
+		asm volatile("bar.sync %0, %1;\n" ::"r"(1 + (int)threadIdx.x / P), "n"(P) : "memory");
 	else __syncthreads();
 }
 
@@ -374,9 +382,11 @@ struct Plan {
 	}
 	// Threads per line of the row tile in every role: a split-1 plan with
 	// B > A gives its middle role (A threads) the load role's B threads, A of
-	// them active, so a line keeps its threads through both stages; 0 (the
-	// role's own count) otherwise.  A CTA holds as many threads either way.
-	static constexpr int ROWW = (S == 1 && B_ > A_) ? B_ : 0;
+	// them active, so a line keeps its threads through both stages; 15, 24 and
+	// 30 threads are rounded up to 16 and 32, so the line stays inside a warp
+	// too; 0 (the role's own count) otherwise.
+	static constexpr int ROWW = (S == 1 && B_ > A_) ? (B_ == 15 ? 16 : B_ == 30 || B_ == 24 ? 32 : B_) : 0;
+	static constexpr int ROWT = ROWW > 0 ? ROWW : TMAX;               // row-tile threads per line
 	// every exchange of to_mid / from_mid takes only warp barriers (a split-1
 	// plan with A > B changes the threads of a line between its stages and
 	// keeps CTA barriers)
@@ -384,7 +394,7 @@ struct Plan {
 	__host__ __device__ static constexpr bool warp_local()
 	{
 		if constexpr (S == 2 || A_ == B_) return Tile::template warp_lines<B>();
-		else return Tile::kWidth == B_ && B_ > A_ && Tile::template warp_lines<B>();
+		else return Tile::kWidth >= B_ && B_ > A_ && Tile::template warp_lines<B>();
 	}
 	template <class Tile>
 	static constexpr int smem_elems()
@@ -405,7 +415,7 @@ struct Plan3 {
 	static constexpr int A = R_, B = R_ * R_;            // load layout: thread j holds x[j + B m], m < A
 	static constexpr int RM = R_, T = B, TMID = B, EMID = R_, TMAX = B;
 	static constexpr int CC = CC_;
-	static constexpr int ROWW = 0;
+	static constexpr int ROWW = 0, ROWT = TMAX;
 	static constexpr bool SMEM_TW = false;
 	static constexpr int TWS = 1, ROW = 1;
 	__device__ __forceinline__ static int mid(int pos, int e) { return pos + B * e; }
@@ -433,11 +443,13 @@ __host__ __device__ constexpr int gcd_ct(int a, int b) { return b == 0 ? a : gcd
 template <class PL>
 __host__ __device__ constexpr int row_lines()
 {
-	constexpr int T = PL::TMAX;
+	constexpr int T = PL::ROWT;
 	constexpr int m = 32 / gcd_ct(T, 32);
 	constexpr int l = (256 / T) / m * m;
 	return l < m ? m : l;
 }
+template <class PL>
+__host__ __device__ constexpr int row_threads() { return row_lines<PL>() * PL::ROWT; }
 // the row tile of a plan
 template <class PL>
 using RowTileOf = RowTile<row_lines<PL>(), PL::ROWW>;
@@ -696,10 +708,10 @@ __device__ __forceinline__ float2 entry_source(const PassArgs& p, int b, int y, 
 // ---------------------------------------------------------------------------
 // Entry row pass: [offset] -> Fourier readout (plane) -> IFT_x.
 template <class PL, class V>
-__global__ void __launch_bounds__(row_lines<PL>() * PL::TMAX)
+__global__ void __launch_bounds__(row_threads<PL>())
 k_entry_rows(const PassArgs p)
 {
-	constexpr int N = PL::N, L = row_lines<PL>(), NT = L * PL::TMAX, NW = Waves<V>::kN;
+	constexpr int N = PL::N, L = row_lines<PL>(), NT = L * PL::ROWT, NW = Waves<V>::kN;
 	using T = RowTileOf<PL>;
 	V* sm = pass_smem<V>();
 	const int tid = threadIdx.x, b = blockIdx.y * NW, row0 = blockIdx.x * L;
@@ -745,7 +757,7 @@ k_entry_rows(const PassArgs p)
 template <class PL, bool READ, class V>
 __device__ __forceinline__ void row_pass_body(const PassArgs& p)
 {
-	constexpr int N = PL::N, L = row_lines<PL>(), NT = L * PL::TMAX;
+	constexpr int N = PL::N, L = row_lines<PL>(), NT = L * PL::ROWT;
 	using T = RowTileOf<PL>;
 	V* sm = pass_smem<V>();
 	const int tid = threadIdx.x, row0 = blockIdx.x * L;
@@ -835,8 +847,8 @@ __device__ __forceinline__ void row_pass_body(const PassArgs& p)
 template <class PL>
 __host__ __device__ constexpr int read_min_blocks()
 {
-	return 65536 / (row_lines<PL>() * PL::TMAX * (PL::RM <= 16 ? 64 : 112)) > 0
-		? 65536 / (row_lines<PL>() * PL::TMAX * (PL::RM <= 16 ? 64 : 112)) : 1;
+	return 65536 / (row_threads<PL>() * (PL::RM <= 16 ? 64 : 112)) > 0
+		? 65536 / (row_threads<PL>() * (PL::RM <= 16 ? 64 : 112)) : 1;
 }
 // Resident CTAs asked of a plain pass of NT threads: the count at 64
 // registers for plans of at most 16 values a thread, at 128 for larger ones.
@@ -849,25 +861,25 @@ __host__ __device__ constexpr int pass_min_blocks()
 	return 65536 / (NT * (PL::RM <= 16 ? 64 : 128)) > 0 ? 65536 / (NT * (PL::RM <= 16 ? 64 : 128)) : 1;
 }
 template <class PL>
-__host__ __device__ constexpr int row_min_blocks() { return pass_min_blocks<PL, row_lines<PL>() * PL::TMAX>(); }
+__host__ __device__ constexpr int row_min_blocks() { return pass_min_blocks<PL, row_threads<PL>()>(); }
 // resident CTAs asked of a pass over wave pairs: at most 128 registers
 template <int NT>
 __host__ __device__ constexpr int pair_min_blocks() { return 65536 / (NT * 128) > 0 ? 65536 / (NT * 128) : 1; }
 template <class PL, class V>
 __host__ __device__ constexpr int row_blocks_sm(bool read)
 {
-	if (Waves<V>::kN == 2) return pair_min_blocks<row_lines<PL>() * PL::TMAX>();
+	if (Waves<V>::kN == 2) return pair_min_blocks<row_threads<PL>()>();
 	return read ? read_min_blocks<PL>() : PL::RM <= 16 ? 0 : row_min_blocks<PL>();
 }
 // plain row pass; the readout planes use k_row_pass_read
 template <class PL, class V>
-__global__ void __launch_bounds__(row_lines<PL>() * PL::TMAX, row_blocks_sm<PL, V>(false))
+__global__ void __launch_bounds__(row_threads<PL>(), row_blocks_sm<PL, V>(false))
 k_row_pass(const PassArgs p)
 {
 	row_pass_body<PL, false, V>(p);
 }
 template <class PL, class V>
-__global__ void __launch_bounds__(row_lines<PL>() * PL::TMAX, row_blocks_sm<PL, V>(true))
+__global__ void __launch_bounds__(row_threads<PL>(), row_blocks_sm<PL, V>(true))
 k_row_pass_read(const PassArgs p)
 {
 	row_pass_body<PL, true, V>(p);
@@ -914,15 +926,16 @@ __host__ __device__ constexpr int col_width(bool narrow)
 // The pass on one tile (grid row blockIdx.y, columns col0 ... col0 + C - 1).
 // SYNC places a CTA barrier between the wave loads and the first transform
 // (which makes a shared twiddle copy filled just before visible).
-// The grating of a plan of at most 16 values a thread is loaded into registers
-// early: for wave pairs before the second DFT, whose arithmetic hides the
-// loads' latency (512^2, 512 waves: 449 -> 424 us), for single waves ahead of
-// everything else; larger plans have no registers to spare.
+// Up to 16 grating values a thread are loaded into registers early: for wave
+// pairs and plans of more values before the second DFT, whose arithmetic hides
+// the loads' latency (512^2 pairs, 512 waves: 449 -> 424 us; 1024^2, 128 waves:
+// 533 -> 503 us), for other single waves ahead of everything else.
 template <class PL, class V, int C, bool READ, int NXC, bool SYNC, class TW>
 __device__ __forceinline__ void col_pass_tile(const PassArgs& p, int col0, const TW& tw, V* sm)
 {
 	constexpr int NW = Waves<V>::kN;
-	constexpr bool EARLY = !READ && PL::EMID <= 16;
+	constexpr int PRE = READ ? 0 : PL::EMID <= 16 ? PL::EMID : 16;   // values loaded early
+	constexpr bool EARLY = PRE > 0;
 	static_assert(!(READ && NW == 2), "images are read out of single waves only");
 	using T = ColTile<C>;
 	const int tid = threadIdx.x, b = blockIdx.y * NW;
@@ -943,17 +956,17 @@ __device__ __forceinline__ void col_pass_tile(const PassArgs& p, int col0, const
 	T::template role<PL::TMID>(tid, cm, pos);
 	const bool mid_live = cm < nval && pos < PL::TMID;
 	const int x = col0 + cm;
-	float2 t[EARLY ? PL::EMID : 1];
+	float2 t[EARLY ? PRE : 1];
 	auto load_t = [&] {
 		if constexpr (EARLY) {
 			if (early && mid_live) {
 				const float2* g = p.mul + o0 + x;
 				#pragma unroll
-				for (int e = 0; e < PL::EMID; e++) t[e] = __ldg(g + PL::mid(pos, e) * nx);
+				for (int e = 0; e < PRE; e++) t[e] = __ldg(g + PL::mid(pos, e) * nx);
 			}
 		}
 	};
-	if constexpr (NW == 1) load_t();   // single waves: ahead of the wait
+	if constexpr (NW == 1 && PL::EMID <= 16) load_t();   // single waves: ahead of the wait
 	pass_wait();
 	// 32-bit offsets within a wave (nx * ny < 2^31): one base pointer per
 	// thread and a row stride, instead of a 64-bit product per element
@@ -967,7 +980,7 @@ __device__ __forceinline__ void col_pass_tile(const PassArgs& p, int col0, const
 	}
 	if constexpr (SYNC) __syncthreads();
 	PL::template to_mid<true, T>(v, sm, tw, tid, [&] {
-		if constexpr (NW == 2) load_t();
+		if constexpr (NW == 2 || PL::EMID > 16) load_t();
 	});
 	if (mid_live) {
 		if constexpr (READ) readout_cols<PL::EMID>(p, b, x, v, [&](int e) { return PL::mid(pos, e); });
@@ -975,7 +988,8 @@ __device__ __forceinline__ void col_pass_tile(const PassArgs& p, int col0, const
 		if (early) {
 			if constexpr (EARLY) {
 				#pragma unroll
-				for (int e = 0; e < PL::EMID; e++) v[e] = cmul(v[e], t[e]);
+				for (int e = 0; e < PL::EMID; e++)
+					v[e] = e < PRE ? cmul(v[e], t[e < PRE ? e : 0]) : cmul(v[e], __ldg(mul + x + PL::mid(pos, e) * nx));
 			}
 		}
 		else if (NW == 1 || o0 == o1) {
@@ -1120,7 +1134,7 @@ cudaError_t launch_entry_t(const PassArgs& p, cudaStream_t s)
 {
 	constexpr int L = row_lines<PL>();
 	constexpr int smem = PL::template smem_elems<RowTileOf<PL>>() * (int)sizeof(V);
-	return launch_k(k_entry_rows<PL, V>, dim3((p.ny + L - 1) / L, wave_rows<V>(p)), L * PL::TMAX, smem, p, s);
+	return launch_k(k_entry_rows<PL, V>, dim3((p.ny + L - 1) / L, wave_rows<V>(p)), L * PL::ROWT, smem, p, s);
 }
 template <class PL, class V>
 cudaError_t launch_row_t(const PassArgs& p, cudaStream_t s)
@@ -1128,8 +1142,8 @@ cudaError_t launch_row_t(const PassArgs& p, cudaStream_t s)
 	constexpr int L = row_lines<PL>();
 	constexpr int smem = PL::template smem_elems<RowTileOf<PL>>() * (int)sizeof(V);
 	const dim3 grid((p.ny + L - 1) / L, wave_rows<V>(p));
-	if (p.plane >= 0) return launch_k(k_row_pass_read<PL, V>, grid, L * PL::TMAX, smem, p, s, true);
-	return launch_k(k_row_pass<PL, V>, grid, L * PL::TMAX, smem, p, s, true);
+	if (p.plane >= 0) return launch_k(k_row_pass_read<PL, V>, grid, L * PL::ROWT, smem, p, s, true);
+	return launch_k(k_row_pass<PL, V>, grid, L * PL::ROWT, smem, p, s, true);
 }
 template <class PL, class V, int C, bool READ, int NXC>
 cudaError_t launch_col_c(const PassArgs& p, cudaStream_t s)

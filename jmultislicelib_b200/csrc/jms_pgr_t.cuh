@@ -10,7 +10,7 @@ namespace jms {
 
 // Rows: IFT_x in place, natural order in and out.
 template <class PL>
-__global__ void __launch_bounds__(row_lines<PL>() * PL::TMAX)
+__global__ void __launch_bounds__(row_threads<PL>())
 k_pgr_rows_inv(float2* work, long long gstride, int ny, const float2* tw)
 {
 	constexpr int N = PL::N, L = row_lines<PL>();
@@ -111,7 +111,7 @@ cudaError_t rows_inv_t(const PgrArgs& p, cudaStream_t s)
 	const dim3 grid((p.ny + L - 1) / L, p.ngr);
 	cudaError_t e = smem_attr(k_pgr_rows_inv<PL>, smem);
 	if (e != cudaSuccess) return e;
-	k_pgr_rows_inv<PL><<<grid, L * PL::TMAX, smem, s>>>(p.out, p.gstride, p.ny, p.twx);
+	k_pgr_rows_inv<PL><<<grid, L * PL::ROWT, smem, s>>>(p.out, p.gstride, p.ny, p.twx);
 	return cudaGetLastError();
 }
 

@@ -1,7 +1,10 @@
 // jms_sizes.h -- supported line lengths and the candidate line plans of each
 // (jms_passes.cuh).  Plan<A, B, C> splits N = A * B (A, B <= 32, radices 2, 3,
 // 4, 5; paired threads when B = 2A); Plan3<R, C> runs N = R^3 in three stages;
-// C is the column-pass tile width.  The first plan of a length is its default;
+// C is the column-pass tile width: 8 columns for plans of more than 16 values a
+// thread, whose wider tiles leave an SM one CTA (per 512 or 256 waves, c16 -> c8:
+// 320 291 -> 219 us, 384 388 -> 357, 480 605 -> 545, 640 514 -> 458, 720 631 -> 586,
+// 768 660 -> 598, 960 545 -> 477, 1024 570 -> 503).  The first plan of a length is its default;
 // JMS_Autotune picks among the candidates by timing them (jms_tune.cpp).
 #pragma once
 #include "jms_kernels.h"
@@ -28,18 +31,18 @@ using P192 = Plan<12, 16, 16>;
 using P240 = Plan<15, 16, 16>;
 using P256a = Plan<16, 16, 16>;
 using P256b = Plan<16, 16, 8>;
-using P320 = Plan<16, 20, 16>;
-using P384 = Plan<16, 24, 16>;
-using P480 = Plan<20, 24, 16>;
+using P320 = Plan<16, 20, 8>;
+using P384 = Plan<16, 24, 8>;
+using P480 = Plan<20, 24, 8>;
 using P512a = Plan<16, 32, 16>;
 using P512b = Plan3<8, 8>;
 using P512c = Plan<16, 32, 8>;
-using P640 = Plan<20, 32, 16>;
-using P720 = Plan<24, 30, 16>;
-using P768 = Plan<24, 32, 16>;
-using P960 = Plan<30, 32, 16>;
-using P1024a = Plan<32, 32, 16>;
-using P1024b = Plan<32, 32, 8>;
+using P640 = Plan<20, 32, 8>;
+using P720 = Plan<24, 30, 8>;
+using P768 = Plan<24, 32, 8>;
+using P960 = Plan<30, 32, 8>;
+using P1024a = Plan<32, 32, 8>;
+using P1024b = Plan<32, 32, 16>;
 using P2048a = Plan<32, 64, 8>;
 using P2048b = Plan<32, 64, 4>;
 
@@ -55,7 +58,7 @@ template <class PL> PlanOps plan_ops_t(int n, const char* name);
 	X(384, P384, "16x24") X(480, P480, "20x24") X(512, P512a, "16x32 pair c16") X(512, P512b, "8x8x8 c8") \
 	X(512, P512c, "16x32 pair c8") \
 	X(640, P640, "20x32") X(720, P720, "24x30") X(768, P768, "24x32") \
-	X(960, P960, "30x32") X(1024, P1024a, "32x32 c16") X(1024, P1024b, "32x32 c8") \
+	X(960, P960, "30x32") X(1024, P1024a, "32x32 c8") X(1024, P1024b, "32x32 c16") \
 	X(2048, P2048a, "32x64 pair c8") X(2048, P2048b, "32x64 pair c4")
 
 // X(length, plan alias): the default (first) plan of every length in

@@ -6,7 +6,8 @@ the same operations on a wave, so a scan in batches large enough for pairs
 equals, bit for bit, the same scan one wave at a time: on square and
 non-square grids, at odd wave counts (the last pair repeats its first wave),
 with pairs of different configurations (odd position counts, one position),
-and with sub-frame gratings.  Plasmon paths, whose draws depend on the batch,
+and with sub-frame gratings.  So do row lines that run under barriers of their
+own (rounded up to 16 or 32 threads, or of two warps).  Plasmon paths, whose draws depend on the batch,
 are compared with the FP64 oracle.
 """
 import numpy as np
@@ -52,7 +53,10 @@ def _setup(J, nx, ny, nobj, nvar, npg=None):
 @pytest.mark.parametrize("nx,ny,npos,npass,npg", [
     (512, 512, 4, 2, None), (512, 512, 5, 1, None), (512, 256, 3, 3, None), (256, 256, 11, 1, None),
     (256, 192, 1, 12, None), (192, 240, 13, 1, None), (128, 128, 19, 3, None), (128, 64, 39, 1, (64, 32)),
-    (64, 64, 39, 1, None), (64, 48, 13, 3, None), (320, 160, 9, 1, None), (16, 16, 300, 1, None)])
+    (64, 64, 39, 1, None), (64, 48, 13, 3, None), (320, 160, 9, 1, None), (16, 16, 300, 1, None),
+    # row lines rounded up to 16 and 32 threads, and of two warps: no pairs, but lines that run by themselves
+    (720, 48, 40, 1, None), (480, 64, 40, 1, None), (384, 48, 40, 1, None), (180, 180, 20, 1, None),
+    (2048, 64, 12, 1, None)])
 def test_pairs_equal_single_waves(J, nx, ny, npos, npass, npg):
     st = _setup(J, nx, ny, 5, 3, npg)
     rng = np.random.default_rng(nx + ny + npos)
