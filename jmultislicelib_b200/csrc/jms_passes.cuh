@@ -453,6 +453,15 @@ __host__ __device__ constexpr int row_threads() { return row_lines<PL>() * PL::R
 // the row tile of a plan
 template <class PL>
 using RowTileOf = RowTile<row_lines<PL>(), PL::ROWW>;
+// rows of a narrow CTA of about 64 threads, for launches that would leave SMs
+// idle (one wave of 512^2: 43 CTAs with live rows, 171 narrow ones)
+template <class PL>
+__host__ __device__ constexpr int narrow_lines()
+{
+	constexpr int m = 32 / gcd_ct(PL::ROWT, 32);
+	constexpr int l = (64 / PL::ROWT) / m * m;
+	return l < m ? m : l;
+}
 
 // ---------------------------------------------------------------------------
 // one wave or two waves per element
@@ -754,11 +763,12 @@ k_entry_rows(const PassArgs p)
 // the variant with the readout code (used at readout planes only, as the
 // kernel k_row_pass_read with launch bounds of its own), so the steps without
 // readout do not carry its registers.
-template <class PL, bool READ, class V>
+// L rows per CTA.
+template <class PL, bool READ, class V, int L>
 __device__ __forceinline__ void row_pass_body(const PassArgs& p)
 {
-	constexpr int N = PL::N, L = row_lines<PL>(), NT = L * PL::ROWT;
-	using T = RowTileOf<PL>;
+	constexpr int N = PL::N, NT = L * PL::ROWT;
+	using T = RowTile<L, PL::ROWW>;
 	V* sm = pass_smem<V>();
 	const int tid = threadIdx.x, row0 = blockIdx.x * L;
 	const int nval = min(L, p.ny - row0);
@@ -872,17 +882,17 @@ __host__ __device__ constexpr int row_blocks_sm(bool read)
 	return read ? read_min_blocks<PL>() : PL::RM <= 16 ? 0 : row_min_blocks<PL>();
 }
 // plain row pass; the readout planes use k_row_pass_read
-template <class PL, class V>
-__global__ void __launch_bounds__(row_threads<PL>(), row_blocks_sm<PL, V>(false))
+template <class PL, class V, int L>
+__global__ void __launch_bounds__(L * PL::ROWT, L == row_lines<PL>() ? row_blocks_sm<PL, V>(false) : 0)
 k_row_pass(const PassArgs p)
 {
-	row_pass_body<PL, false, V>(p);
+	row_pass_body<PL, false, V, L>(p);
 }
 template <class PL, class V>
 __global__ void __launch_bounds__(row_threads<PL>(), row_blocks_sm<PL, V>(true))
 k_row_pass_read(const PassArgs p)
 {
-	row_pass_body<PL, true, V>(p);
+	row_pass_body<PL, true, V, row_lines<PL>()>(p);
 }
 
 // Live rows of a column-pass thread as a bit mask: bit m is set when row
@@ -1143,7 +1153,13 @@ cudaError_t launch_row_t(const PassArgs& p, cudaStream_t s)
 	constexpr int smem = PL::template smem_elems<RowTileOf<PL>>() * (int)sizeof(V);
 	const dim3 grid((p.ny + L - 1) / L, wave_rows<V>(p));
 	if (p.plane >= 0) return launch_k(k_row_pass_read<PL, V>, grid, L * PL::ROWT, smem, p, s, true);
-	return launch_k(k_row_pass<PL, V>, grid, L * PL::ROWT, smem, p, s, true);
+	if constexpr (Waves<V>::kN == 1 && PL::N >= 256) {
+		constexpr int LN = narrow_lines<PL>();
+		constexpr int smem_n = PL::template smem_elems<RowTile<LN, PL::ROWW>>() * (int)sizeof(V);
+		if ((long long)grid.x * p.nwave < kSMs)
+			return launch_k(k_row_pass<PL, V, LN>, dim3((p.ny + LN - 1) / LN, p.nwave), LN * PL::ROWT, smem_n, p, s, true);
+	}
+	return launch_k(k_row_pass<PL, V, L>, grid, L * PL::ROWT, smem, p, s, true);
 }
 template <class PL, class V, int C, bool READ, int NXC>
 cudaError_t launch_col_c(const PassArgs& p, cudaStream_t s)
