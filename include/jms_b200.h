@@ -152,7 +152,9 @@ int JMS_ScanGPU(int npos, const float* pos, float dz, int npass, const int* vars
  * d_out_int is double [npos][ndetslc][ndet] and is accumulated into. */
 int JMS_ScanGPUDevice(int npos, const float* d_pos, float dz, int npass, const int* varseq, double* d_out_int,
 	float* d_out_bin, int bin);
-/* Probe positions processed together in one pass sequence (default 32). */
+/* Probe positions processed together in one pass sequence (default 32).  With
+ * pass fusion on, scans of small grids put more waves into a launch, up to
+ * 64 MB of them. */
 int JMS_SetScanBatch(int nwave);
 /* Frozen-phonon configurations in one launch (no counterpart in the
  * reference, whose GPUMultislice runs one wave per call,
