@@ -13,11 +13,8 @@
 // weights [O][C].  The ReLU mask of a layer is its stored output (y > 0).
 #include "../../include/jms_b200.h"
 
-#include <cooperative_groups.h>
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
-
-namespace cg = cooperative_groups;
 
 namespace {
 
@@ -29,7 +26,11 @@ __device__ __forceinline__ float bf(const __nv_bfloat16 v) { return __bfloat162f
 // keeps the reuse of a value in registers.  Batch 256, ten 16 x 16 channels, all
 // layers of a training step, against one thread per output (or per sum) reading
 // every operand from global memory: forward 92 -> 54 us, weight gradients
-// 152 -> 69, data gradients 102 -> 48; still mostly waiting on global loads.
+// 152 -> 82, data gradients 102 -> 55; still mostly waiting on global loads.
+// Every sum has one order of its FP32 additions, given at its kernel, that no
+// tile, chunk or grid changes: Adam divides a gradient by its own magnitude, so
+// in a few training steps another rounding of a gradient near zero becomes 1e-4
+// of a bias.
 
 // y[b][co][oy][ox] = relu(bias[co] + sum_ci,ky,kx w[co][ci][ky][kx] x[b][ci][2oy-1+ky][2ox-1+kx])
 // A CTA makes PT output pixels (flattened b, oy, ox) of 16 output channels; 4 PT
@@ -100,191 +101,178 @@ __global__ void __launch_bounds__(kNnThr) k_conv_fwd(const __nv_bfloat16* __rest
 // with g = dy * (y > 0) when relu.  A thread makes the 2 x 2 block of input
 // pixels at (2a, 2b') of one channel, which sees the four outputs (a, b'),
 // (a, b'+1), (a+1, b'), (a+1, b'+1): nine products per output channel and no
-// masked taps.  A CTA takes 16 blocks x 16 input channels, output channels in
-// chunks of kBwdCo; a warp takes two blocks, its half warps every other output
-// channel, so a weight read from shared memory serves two blocks and the 32
-// lanes read 32 banks.
-constexpr int kBwdCo = 32;
+// masked taps.  A CTA takes 16 blocks x 16 input channels and output channels in
+// chunks of kBwdCo.  A sum runs tap by tap (ky, kx ascending), over the output
+// channels within a tap: four sweeps over the channels, one per tap of the
+// pixel that has four.  Up to kBwdCo output channels are staged once for all
+// four.
+constexpr int kBwdCo = 64;
 template <class I>
 __global__ void __launch_bounds__(kNnThr) k_conv_bwd_data(const float* __restrict__ dy,
 	const __nv_bfloat16* __restrict__ y, const __nv_bfloat16* __restrict__ w, float* __restrict__ dx, int B, int Ci,
 	int H, int W, int Co, int relu)
 {
 	__shared__ __align__(16) float gs[kBwdCo][16][4];
-	__shared__ float ws[kBwdCo][16][9];                // a stride of 9 keeps the 16 channels on distinct banks
+	__shared__ __nv_bfloat16 ws[kBwdCo][9][16];
 	const int Ho = H / 2, Wo = W / 2, hw = Ho * Wo;
 	const I npix = (I)B * hw, pix0 = (I)blockIdx.x * 16;
-	const int ci0 = blockIdx.y * 16, c = threadIdx.x % 16, half = (threadIdx.x / 16) % 2, q0 = 2 * (threadIdx.x / 32);
-	int bb[2], aa[2], dd[2];
-	bool right[2], down[2];
-	float o[2][4];
-	#pragma unroll
-	for (int u = 0; u < 2; u++) {
-		const I pix = pix0 + q0 + u;
-		bb[u] = (int)(pix / hw);
-		const int r = (int)(pix - (I)bb[u] * hw);
-		aa[u] = r / Wo;
-		dd[u] = r % Wo;
-		right[u] = dd[u] + 1 < Wo;
-		down[u] = aa[u] + 1 < Ho;
-		#pragma unroll
-		for (int k = 0; k < 4; k++) o[u][k] = 0.f;
-	}
-	for (int k0 = 0; k0 < Co; k0 += kBwdCo) {
-		const int nk = min(kBwdCo, Co - k0);
-		__syncthreads();
-		#pragma unroll
-		for (int i = threadIdx.x; i < kBwdCo * 64; i += kNnThr) {
-			const int k = i / 64, h = i % 4;
-			const I pi = pix0 + (i / 4) % 16;
-			const int bi = (int)(pi / hw), ri = (int)(pi - (I)bi * hw), ai = ri / Wo + (h >> 1), di = ri % Wo + (h & 1);
-			float g = 0.f;
-			if (k < nk && pi < npix && ai < Ho && di < Wo) {
-				const long long o = (((long long)bi * Co + k0 + k) * Ho + ai) * Wo + di;
-				g = dy[o];
-				if (relu && !(bf(y[o]) > 0.f)) g = 0.f;
+	const int ci0 = blockIdx.y * 16, c = threadIdx.x % 16, q = threadIdx.x / 16;
+	const I pix = pix0 + q;
+	const int b = (int)(pix / hw), p = (int)(pix - (I)b * hw), a = p / Wo, d = p - a * Wo;
+	const bool right = d + 1 < Wo, down = a + 1 < Ho;
+	float o0 = 0.f, o1 = 0.f, o2 = 0.f, o3 = 0.f;
+	for (int sweep = 0; sweep < 4; sweep++) {
+		for (int k0 = 0; k0 < Co; k0 += kBwdCo) {
+			const int nk = min(kBwdCo, Co - k0);
+			if (sweep == 0 || Co > kBwdCo) {
+				__syncthreads();
+				#pragma unroll 8
+				for (int i = threadIdx.x; i < nk * 64; i += kNnThr) {
+					const int k = i / 64, h = i % 4;
+					const I pi = pix0 + (i / 4) % 16;
+					const int bi = (int)(pi / hw), ri = (int)(pi - (I)bi * hw), ai = ri / Wo + (h >> 1), di = ri % Wo + (h & 1);
+					float g = 0.f;
+					if (pi < npix && ai < Ho && di < Wo) {
+						const long long o = (((long long)bi * Co + k0 + k) * Ho + ai) * Wo + di;
+						g = dy[o];
+						if (relu && !(bf(y[o]) > 0.f)) g = 0.f;
+					}
+					gs[k][(i / 4) % 16][h] = g;
+				}
+				#pragma unroll 12
+				for (int i = threadIdx.x; i < nk * 144; i += kNnThr) {
+					const int k = i / 144, r = i - 144 * k;
+					if (ci0 + r / 9 < Ci) ws[k][r % 9][r / 9] = w[((long long)(k0 + k) * Ci + ci0) * 9 + r];
+				}
+				__syncthreads();
 			}
-			gs[k][(i / 4) % 16][h] = g;
-		}
-		#pragma unroll 6
-		for (int i = threadIdx.x; i < kBwdCo * 144; i += kNnThr) {
-			const int k = i / 144, r = i - 144 * k;
-			ws[k][r / 9][r % 9] = (k < nk && ci0 + r / 9 < Ci) ? bf(w[((long long)(k0 + k) * Ci + ci0) * 9 + r]) : 0.f;
-		}
-		__syncthreads();
-		#pragma unroll 2
-		for (int k = half; k < nk; k += 2) {
-			float t[9];
-			#pragma unroll
-			for (int i = 0; i < 9; i++) t[i] = ws[k][c][i];
-			#pragma unroll
-			for (int u = 0; u < 2; u++) {
-				const float4 g = *reinterpret_cast<const float4*>(gs[k][q0 + u]);   // (a,b'), (a,b'+1), (a+1,b'), (a+1,b'+1)
-				o[u][0] = fmaf(g.x, t[4], o[u][0]);
-				o[u][1] = fmaf(g.x, t[5], o[u][1]);
-				o[u][2] = fmaf(g.x, t[7], o[u][2]);
-				o[u][3] = fmaf(g.x, t[8], o[u][3]);
-				if (right[u]) { o[u][1] = fmaf(g.y, t[3], o[u][1]); o[u][3] = fmaf(g.y, t[6], o[u][3]); }
-				if (down[u]) { o[u][2] = fmaf(g.z, t[1], o[u][2]); o[u][3] = fmaf(g.z, t[2], o[u][3]); }
-				if (right[u] && down[u]) o[u][3] = fmaf(g.w, t[0], o[u][3]);
+			auto tap = [&](int k, int t) { return bf(ws[k][t][c]); };
+			auto grad = [&](int k) { return *reinterpret_cast<const float4*>(gs[k][q]); };   // (a,b'), (a,b'+1), (a+1,b'), (a+1,b'+1)
+			if (sweep == 0) {
+				#pragma unroll 4
+				for (int k = 0; k < nk; k++) {
+					const float4 g = grad(k);
+					o0 = fmaf(g.x, tap(k, 4), o0);
+					if (right) o1 = fmaf(g.y, tap(k, 3), o1);
+					if (down) o2 = fmaf(g.z, tap(k, 1), o2);
+					if (right && down) o3 = fmaf(g.w, tap(k, 0), o3);
+				}
+			}
+			else if (sweep == 1) {
+				#pragma unroll 4
+				for (int k = 0; k < nk; k++) {
+					const float4 g = grad(k);
+					o1 = fmaf(g.x, tap(k, 5), o1);
+					o2 = fmaf(g.x, tap(k, 7), o2);
+					if (down) o3 = fmaf(g.z, tap(k, 2), o3);
+				}
+			}
+			else if (sweep == 2) {
+				#pragma unroll 8
+				for (int k = 0; k < nk; k++)
+					if (right) o3 = fmaf(gs[k][q][1], tap(k, 6), o3);
+			}
+			else {
+				#pragma unroll 8
+				for (int k = 0; k < nk; k++) o3 = fmaf(gs[k][q][0], tap(k, 8), o3);
 			}
 		}
 	}
-	#pragma unroll
-	for (int u = 0; u < 2; u++) {
-		#pragma unroll
-		for (int k = 0; k < 4; k++) o[u][k] += __shfl_xor_sync(0xffffffffu, o[u][k], 16);
-	}
-	const int u = half;        // each half warp stores one of the two blocks
-	const I pix = pix0 + q0 + u;
 	if (pix >= npix || ci0 + c >= Ci) return;
-	float* out = dx + (((long long)(u ? bb[1] : bb[0]) * Ci + ci0 + c) * H + 2 * (u ? aa[1] : aa[0])) * W +
-		2 * (u ? dd[1] : dd[0]);
-	out[0] = u ? o[1][0] : o[0][0];
-	out[1] = u ? o[1][1] : o[0][1];
-	out[W] = u ? o[1][2] : o[0][2];
-	out[W + 1] = u ? o[1][3] : o[0][3];
+	float* out = dx + (((long long)b * Ci + ci0 + c) * H + 2 * a) * W + 2 * d;
+	out[0] = o0;
+	out[1] = o1;
+	out[W] = o2;
+	out[W + 1] = o3;
 }
 
 // dw[co][ci][ky][kx] = sum_b,oy,ox g[b][co][oy][ox] x[b][ci][iy][ix]; db[co] = sum g.
-// A CTA takes four output channels and one input channel: a thread reads an
-// output pixel's nine taps once for the four channels.  The pixels are split
-// over the CTAs of a cluster (gridDim.z = the cluster), whose sums the first
-// one adds in rank order; the CTAs of ci = 0 also make db.
-constexpr int kBwCo = 4, kBwSums = 9 * kBwCo + kBwCo, kBwMaxSplit = 8;
+// A CTA takes four output channels, one input channel and one row ky of taps: a
+// thread reads an output pixel's three taps once for the four channels, and the
+// three rows give the first layers, which have the most pixels and the fewest
+// channels, CTAs for every SM.  Four pixels' loads are in flight at once (first
+// layer 37 -> 26 us).  A sum runs over a thread's pixels (t, t + 256,
+// ...), then over the lanes of a warp in halves, then over the warps.  The CTAs
+// of ci = 0, ky = 1 also make db.
+constexpr int kBwCo = 4, kBwSums = 4 * kBwCo;
 template <class I>
 __global__ void __launch_bounds__(kNnThr) k_conv_bwd_weight(const __nv_bfloat16* __restrict__ x,
 	const float* __restrict__ dy, const __nv_bfloat16* __restrict__ y, float* __restrict__ dw, float* __restrict__ db,
 	int B, int Ci, int H, int W, int Co, int relu)
 {
 	__shared__ float red[kNnThr / 32][kBwSums];
-	__shared__ float sums[kBwSums];
-	const int ci = blockIdx.x, co0 = blockIdx.y * kBwCo, rank = blockIdx.z, nrank = gridDim.z;
+	const int ci = blockIdx.x, co0 = blockIdx.y * kBwCo, ky = blockIdx.z;
 	const int Ho = H / 2, Wo = W / 2, hw = Ho * Wo;
-	const I n = (I)B * hw, per = (n + nrank - 1) / nrank, i1 = n < (rank + 1) * per ? n : (rank + 1) * per;
-	float acc[kBwCo][9], gb[kBwCo];
+	const I n = (I)B * hw;
+	float a[kBwSums];        // sum 4 c + kx of channel c, and 4 c + 3 its sum of g
 	#pragma unroll
-	for (int c = 0; c < kBwCo; c++) {
-		gb[c] = 0.f;
+	for (int k = 0; k < kBwSums; k++) a[k] = 0.f;
+	// pixel (b, oy, ox) of i and its step of 256 pixels, carried instead of divided
+	int b = (int)threadIdx.x / hw, oy = (int)threadIdx.x % hw / Wo, ox = (int)threadIdx.x % hw % Wo;
+	const int sb = kNnThr / hw, sy = kNnThr % hw / Wo, sx = kNnThr % hw % Wo;
+	constexpr int U = 4;     // pixels whose loads are in flight together
+	for (I i = threadIdx.x; i < n; i += U * kNnThr) {
+		float v[U][3], g[U][kBwCo];
+		bool top[U], left[U], live[U];
 		#pragma unroll
-		for (int t = 0; t < 9; t++) acc[c][t] = 0.f;
-	}
-	#pragma unroll 2
-	for (I i = rank * per + threadIdx.x; i < i1; i += kNnThr) {
-		const int b = (int)(i / hw), p = (int)(i - (I)b * hw), oy = p / Wo, ox = p - oy * Wo;
-		const __nv_bfloat16* xp = x + ((long long)b * Ci + ci) * H * W;
-		float v[9];
-		#pragma unroll
-		for (int t = 0; t < 9; t++) {
-			const int iy = 2 * oy - 1 + t / 3, ix = 2 * ox - 1 + t % 3;
-			v[t] = (iy >= 0 && ix >= 0) ? bf(xp[iy * W + ix]) : 0.f;
-		}
-		#pragma unroll
-		for (int c = 0; c < kBwCo; c++) {
-			float g = 0.f;
-			if (co0 + c < Co) {
-				const long long o = ((long long)b * Co + co0 + c) * hw + p;
-				g = dy[o];
-				if (relu && !(bf(y[o]) > 0.f)) g = 0.f;
-			}
-			gb[c] += g;
+		for (int u = 0; u < U; u++) {
+			const int p = oy * Wo + ox, iy = 2 * oy - 1 + ky, ix = 2 * ox - 1;
+			live[u] = u == 0 || n - i > u * kNnThr;
+			top[u] = live[u] && iy >= 0;
+			left[u] = top[u] && ix >= 0;
+			const __nv_bfloat16* xp = x + (((long long)b * Ci + ci) * H + iy) * W + ix;
+			v[u][0] = left[u] ? bf(xp[0]) : 0.f;
+			v[u][1] = top[u] ? bf(xp[1]) : 0.f;
+			v[u][2] = top[u] ? bf(xp[2]) : 0.f;
+			const long long o = ((long long)b * Co + co0) * hw + p;
 			#pragma unroll
-			for (int t = 0; t < 9; t++)
-				if (!((t < 3 && oy == 0) || (t % 3 == 0 && ox == 0))) acc[c][t] = fmaf(g, v[t], acc[c][t]);
+			for (int c = 0; c < kBwCo; c++) {
+				const bool in = live[u] && co0 + c < Co;
+				g[u][c] = in ? dy[o + (long long)c * hw] : 0.f;
+				if (relu && in && !(bf(y[o + (long long)c * hw]) > 0.f)) g[u][c] = 0.f;
+			}
+			ox += sx;
+			oy += sy + (ox >= Wo);
+			ox -= ox >= Wo ? Wo : 0;
+			b += sb + (oy >= Ho);
+			oy -= oy >= Ho ? Ho : 0;
+		}
+		#pragma unroll
+		for (int u = 0; u < U; u++) {
+			#pragma unroll
+			for (int c = 0; c < kBwCo; c++) {
+				if (left[u]) a[4 * c] = fmaf(g[u][c], v[u][0], a[4 * c]);
+				if (top[u]) a[4 * c + 1] = fmaf(g[u][c], v[u][1], a[4 * c + 1]);
+				if (top[u]) a[4 * c + 2] = fmaf(g[u][c], v[u][2], a[4 * c + 2]);
+				if (live[u]) a[4 * c + 3] += g[u][c];
+			}
 		}
 	}
+	// 16 sums at once: each step halves the sums a lane holds, so lane 2 k ends
+	// with sum k
 	const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-	// 32 sums at once: each step halves the sums a lane holds, so lane k ends
-	// with sum k after 31 shuffles
-	float a[32];
 	#pragma unroll
-	for (int k = 0; k < 32; k++) a[k] = acc[k / 9][k % 9];
-	#pragma unroll
-	for (int h = 16; h > 0; h >>= 1) {
+	for (int h = 16; h > 1; h >>= 1) {
 		const bool up = lane & h;
 		#pragma unroll
-		for (int k = 0; k < h; k++) {
-			const float keep = up ? a[k + h] : a[k], send = up ? a[k] : a[k + h];
+		for (int k = 0; k < h / 2; k++) {
+			const float keep = up ? a[k + h / 2] : a[k], send = up ? a[k] : a[k + h / 2];
 			a[k] = keep + __shfl_xor_sync(0xffffffffu, send, h);
 		}
 	}
-	red[warp][lane] = a[0];
-	auto warp_red = [&](float s, int k) {
-		#pragma unroll
-		for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-		if (lane == 0) red[warp][k] = s;
-	};
-	static_assert(9 * kBwCo >= 32, "the transposing sum takes the first 32");
-	#pragma unroll
-	for (int k = 32; k < 9 * kBwCo; k++) warp_red(acc[k / 9][k % 9], k);
-	if (ci == 0) {
-		#pragma unroll
-		for (int c = 0; c < kBwCo; c++) warp_red(gb[c], 9 * kBwCo + c);
-	}
+	a[0] += __shfl_xor_sync(0xffffffffu, a[0], 1);
+	if (!(lane & 1)) red[warp][lane >> 1] = a[0];
 	__syncthreads();
 	const int k = threadIdx.x;
-	const bool mine = k < (ci == 0 ? kBwSums : 9 * kBwCo);
-	if (mine) {
-		float s = 0.f;
-		#pragma unroll
-		for (int q = 0; q < kNnThr / 32; q++) s += red[q][k];
-		sums[k] = s;
-	}
-	cg::cluster_group cl = cg::this_cluster();
-	cl.sync();
-	if (rank == 0 && mine) {
-		float s = sums[k];
-		for (int r = 1; r < nrank; r++) s += *cl.map_shared_rank(&sums[k], r);
-		if (k < 9 * kBwCo) {
-			const int co = co0 + k / 9;
-			if (co < Co) dw[((long long)co * Ci + ci) * 9 + k % 9] = s;
-		}
-		else if (co0 + k - 9 * kBwCo < Co) db[co0 + k - 9 * kBwCo] = s;
-	}
-	cl.sync();   // the other CTAs' sums are read before they leave
+	if (k >= kBwSums || co0 + k / 4 >= Co) return;
+	float s = 0.f;
+	#pragma unroll
+	for (int q = 0; q < kNnThr / 32; q++) s += red[q][k];
+	if (k % 4 < 3) dw[((long long)(co0 + k / 4) * Ci + ci) * 9 + 3 * ky + k % 4] = s;
+	else if (ci == 0 && ky == 1) db[co0 + k / 4] = s;
 }
 
-// out[b][o] = bl[o] + sum_c wl[o][c] mean_hw h[b][c][hw]; four threads per output
+// out[b][o] = bl[o] + sum_c wl[o][c] mean_hw h[b][c][hw], summed in that order
 __global__ void k_pool_linear_fwd(const __nv_bfloat16* __restrict__ h, const float* __restrict__ wl,
 	const float* __restrict__ bl, float* __restrict__ out, int B, int C, int HW, int O)
 {
@@ -297,17 +285,11 @@ __global__ void k_pool_linear_fwd(const __nv_bfloat16* __restrict__ h, const flo
 		pooled[c] = s / (float)HW;
 	}
 	__syncthreads();
-	const int part = threadIdx.x & 3;
-	for (int o0 = 0; o0 < O; o0 += blockDim.x / 4) {   // uniform trips: the shuffles need whole warps
-		const int o = o0 + threadIdx.x / 4;
-		float s = 0.f;
-		if (o < O) {
-			#pragma unroll 4
-			for (int c = part; c < C; c += 4) s = fmaf(__ldg(wl + (long long)o * C + c), pooled[c], s);
-		}
-		s += __shfl_xor_sync(0xffffffffu, s, 1);
-		s += __shfl_xor_sync(0xffffffffu, s, 2);
-		if (o < O && part == 0) out[(long long)b * O + o] = bl[o] + s;
+	for (int o = threadIdx.x; o < O; o += blockDim.x) {
+		float s = bl[o];
+		#pragma unroll 16
+		for (int c = 0; c < C; c++) s = fmaf(__ldg(wl + (long long)o * C + c), pooled[c], s);
+		out[(long long)b * O + o] = s;
 	}
 }
 
@@ -324,31 +306,44 @@ __global__ void k_pool_linear_bwd_data(const float* __restrict__ wl, const float
 	dh[i] = s / (float)HW;
 }
 
-// dwl[o][c] = sum_b dout[b][o] pooled[b][c]; dbl[o] = sum_b dout[b][o]; a warp
-// per (o, c | bias), its lanes over the batch (as one thread per sum walking
-// the batch it took 101 us at 256 x 64 x 30, all of it latency)
+// dwl[o][c] = sum_b dout[b][o] pooled[b][c]; dbl[o] = sum_b dout[b][o], summed
+// in the order of b.  A CTA makes 16 x 16 sums (the bias is column C, whose
+// factor is 1) and stages their factors for kPlB images at once, so a sum waits
+// for memory once per chunk (256 x 64 x 30: 8 us; reading both factors in its
+// loop, 101 us).
+constexpr int kPlB = 256;
 __global__ void __launch_bounds__(kNnThr) k_pool_linear_bwd_weight(const __nv_bfloat16* __restrict__ h,
 	const float* __restrict__ dout, float* __restrict__ dwl, float* __restrict__ dbl, int B, int C, int HW, int O)
 {
-	const int i = (blockIdx.x * kNnThr + threadIdx.x) / 32, lane = threadIdx.x & 31;
-	if (i >= O * (C + 1)) return;
-	const int o = i / (C + 1), c = i % (C + 1);
+	__shared__ float ps[kPlB][16], gs[kPlB][16];
+	const int nct = C / 16 + 1, c0 = blockIdx.x % nct * 16, o0 = blockIdx.x / nct * 16;   // C + 1 columns
+	const int tc = threadIdx.x % 16, to = threadIdx.x / 16, c = c0 + tc, o = o0 + to;
 	float s = 0.f;
-	#pragma unroll 4
-	for (int b = lane; b < B; b += 32) {
-		const float g = dout[(long long)b * O + o];
-		if (c == C) { s += g; continue; }
-		const __nv_bfloat16* hp = h + ((long long)b * C + c) * HW;
-		float p = 0.f;
-		for (int k = 0; k < HW; k++) p += bf(hp[k]);
-		s = fmaf(g, p / (float)HW, s);
+	for (int b0 = 0; b0 < B; b0 += kPlB) {
+		const int nb = min(kPlB, B - b0);
+		__syncthreads();
+		#pragma unroll 8
+		for (int k = to; k < nb; k += kNnThr / 16) gs[k][tc] = o0 + tc < O ? dout[(long long)(b0 + k) * O + o0 + tc] : 0.f;
+		const __nv_bfloat16* hp = h + ((long long)b0 * C + c) * HW;
+		if (c >= C || HW == 1) {   // independent loads
+			#pragma unroll 8
+			for (int k = to; k < nb; k += kNnThr / 16) ps[k][tc] = c < C ? bf(hp[(long long)k * C]) : 1.f;
+		}
+		else {
+			for (int k = to; k < nb; k += kNnThr / 16) {
+				float p = 0.f;
+				#pragma unroll 4
+				for (int i = 0; i < HW; i++) p += bf(hp[(long long)k * C * HW + i]);
+				ps[k][tc] = p / (float)HW;
+			}
+		}
+		__syncthreads();
+		#pragma unroll 16
+		for (int k = 0; k < nb; k++) s = fmaf(gs[k][to], ps[k][tc], s);
 	}
-	#pragma unroll
-	for (int q = 16; q > 0; q >>= 1) s += __shfl_xor_sync(0xffffffffu, s, q);
-	if (lane == 0) {
-		if (c == C) dbl[o] = s;
-		else dwl[(long long)o * C + c] = s;
-	}
+	if (o >= O || c > C) return;
+	if (c == C) dbl[o] = s;
+	else dwl[(long long)o * C + c] = s;
 }
 
 // dout = 2 (out - t) / n; loss partial sums of (out - t)^2 / n (atomic into *loss)
@@ -483,25 +478,8 @@ int JMS_NnConvBackward(const void* x, const void* w, const void* y, const float*
 	if (dx)
 		(big ? k_conv_bwd_data<long long> : k_conv_bwd_data<int>)<<<dim3((unsigned)((npix + 15) / 16), (unsigned)((Ci + 15) / 16)), kNnThr, 0, s>>>(dy,
 			(const __nv_bfloat16*)y, (const __nv_bfloat16*)w, dx, B, Ci, H, W, Co, relu);
-	// pixels over up to eight CTAs where the channel pairs alone leave SMs idle
-	// and every thread still has two pixels
-	const unsigned ncq = (unsigned)((Co + kBwCo - 1) / kBwCo);
-	unsigned split = 1;
-	while (split < kBwMaxSplit && (long long)Ci * ncq * split < 296 && npix >= 4LL * kNnThr * split) split *= 2;
-	cudaLaunchConfig_t cfg = {};
-	cfg.gridDim = dim3((unsigned)Ci, ncq, split);
-	cfg.blockDim = dim3(kNnThr);
-	cfg.stream = s;
-	cudaLaunchAttribute at;
-	at.id = cudaLaunchAttributeClusterDimension;
-	at.val.clusterDim.x = 1;
-	at.val.clusterDim.y = 1;
-	at.val.clusterDim.z = split;
-	cfg.attrs = &at;
-	cfg.numAttrs = 1;
-	if (cudaLaunchKernelEx(&cfg, big ? k_conv_bwd_weight<long long> : k_conv_bwd_weight<int>, (const __nv_bfloat16*)x, dy, (const __nv_bfloat16*)y, dw, db, B, Ci,
-		H, W, Co, relu) != cudaSuccess)
-		return 1;
+	(big ? k_conv_bwd_weight<long long> : k_conv_bwd_weight<int>)<<<dim3((unsigned)Ci, (unsigned)((Co + kBwCo - 1) / kBwCo), 3),
+		kNnThr, 0, s>>>((const __nv_bfloat16*)x, dy, (const __nv_bfloat16*)y, dw, db, B, Ci, H, W, Co, relu);
 	return ok(s);
 }
 
@@ -523,8 +501,8 @@ int JMS_NnPoolLinearBackward(const void* h, const float* wl, const float* dout, 
 		const long long n = (long long)B * C * HW;
 		k_pool_linear_bwd_data<<<nblk(n, 256), 256, 0, s>>>(wl, dout, dh, B, C, HW, O);
 	}
-	k_pool_linear_bwd_weight<<<nblk(32LL * O * (C + 1), kNnThr), kNnThr, 0, s>>>((const __nv_bfloat16*)h, dout, dwl, dbl,
-		B, C, HW, O);
+	k_pool_linear_bwd_weight<<<(unsigned)(C / 16 + 1) * (unsigned)((O + 15) / 16), kNnThr, 0, s>>>((const __nv_bfloat16*)h,
+		dout, dwl, dbl, B, C, HW, O);
 	return ok(s);
 }
 

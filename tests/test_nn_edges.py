@@ -1,10 +1,9 @@
 """Surrogate convolutions and pooling at the edges of their tiles.
 
 Channel counts that are not multiples of the kernels' groups (16 output
-channels, chunks of 8 input and 16 output channels, four output channels of
-the weight gradient), pixel counts below, at and above one tile, non-square
-images down to 2 x 2, and pixel splits over a cluster, against the FP64
-restatement (oracle/nn_oracle.py).  Bounds: an FP32 sum of n products is
+channels, chunks of 8 input channels, four output channels of the weight
+gradient), pixel counts below, at and above one tile, and non-square images
+down to 2 x 2, against the FP64 restatement (oracle/nn_oracle.py).  Bounds: an FP32 sum of n products is
 within n * 2^-24 of the sum of their magnitudes; the forward result is then
 rounded to BF16 (2^-8 of the value).
 """
