@@ -153,8 +153,9 @@ int JMS_ScanGPU(int npos, const float* pos, float dz, int npass, const int* vars
 int JMS_ScanGPUDevice(int npos, const float* d_pos, float dz, int npass, const int* varseq, double* d_out_int,
 	float* d_out_bin, int bin);
 /* Probe positions processed together in one pass sequence (default 32).  With
- * pass fusion on, scans of small grids put more waves into a launch, up to
- * 64 MB of them. */
+ * pass fusion on and a batch of at least the default, scans of small grids put
+ * more waves into a launch, up to 64 MB of them and 4096; a smaller batch
+ * bounds the waves in flight. */
 int JMS_SetScanBatch(int nwave);
 /* Frozen-phonon configurations in one launch (no counterpart in the
  * reference, whose GPUMultislice runs one wave per call,

@@ -1166,9 +1166,12 @@ int JmsB200::ScanGPUDevice(int npos, const float* d_pos, float dz, int npass, co
 	// kMergePoints wave points (64 MB, which stays in L2): 32 waves of 128^2 fill
 	// a fifth of the GPU and run at launch latency.  Wave k * np + p is position p
 	// in configuration k.  Needs no plasmon paths and grating offsets within int
-	// range.  At most 4096 waves, which bounds the per-wave tables and sums.
+	// range.  At most 4096 waves, which bounds the per-wave tables and sums.  A
+	// batch below the default is a caller's bound on the waves in flight: it is
+	// kept.
 	constexpr long long kMergePoints = 1LL << 23, kMergeWaves = 4096;
-	const int Wm = (int)std::max<long long>(B, std::min(kMergeWaves, kMergePoints / std::max(1LL, (long long)nx_ * ny_)));
+	const int Wm = B < kDefaultBatch ? B
+		: (int)std::max<long long>(B, std::min(kMergeWaves, kMergePoints / std::max(1LL, (long long)nx_ * ny_)));
 	const long long pool = slcoffset_.empty() ? 0
 		: slcoffset_.back() + (long long)nvarslc_.back() * npgx_ * npgy_;
 	// A stream capture keeps the sequential form: the fused form uploads its

@@ -244,7 +244,8 @@ private:
 	float *d_dif_ = nullptr, *d_img_ = nullptr, *d_dif_avg_ = nullptr, *d_img_avg_ = nullptr;
 	float2 *d_wff_ = nullptr, *d_wfr_ = nullptr, *d_wff_avg_ = nullptr, *d_wfr_avg_ = nullptr;
 	float weight_imgavg_ = 0.f, weight_wavavg_ = 0.f;
-	int scan_batch_ = 32;
+	static constexpr int kDefaultBatch = 32;
+	int scan_batch_ = kDefaultBatch;
 	int descan_on_ = 0, descan_x_ = 0, descan_y_ = 0;
 	int timing_on_ = 0;
 	const PlanOps* prow_ = nullptr;  // plan of the row / entry passes (length nx)

@@ -1,0 +1,72 @@
+"""Batches and configurations of a scan put together in one launch.
+
+With the default batch or a larger one, a scan of a small grid puts positions
+and configurations together up to 64 MB of waves per launch (at 256^2: 128
+waves).  Checked against the same scan with one launch sequence per batch and
+configuration (JMS_SetPassFusion(0)), whose waves are the same: the detector
+sums agree to the last place of their FP32 results (2^-23) and the binned patterns to
+the order of their float atomics.
+"""
+import numpy as np
+import pytest
+
+from tests import golden_cases as G
+from tests import product_cases as PC
+
+pytestmark = pytest.mark.gpu
+GPU = 2
+
+
+@pytest.fixture()
+def J():
+    import jmultislicelib_b200 as jb
+
+    j = jb.JMS()
+    yield j
+    j.L.JMS_SetScanBatch(32)
+    j.L.JMS_SetPassFusion(1)
+
+
+def _setup(J, n, nobj=5, nvar=3, flags=G.INT):
+    a = 0.045 * n
+    J.cleanup()
+    J.set_high_tension(300.0)
+    J.set_grid(n, n, a, a, 0.4)
+    pro = J.calc_propagator(0.19525, 0.0, 0.0, 1)
+    probe = J.calc_probe(22.0)
+    pgr = PC.synthetic_specimen(n, n, 2, nvar, 3 + n)
+    assert J.setup(GPU, [nvar, nvar], np.arange(nobj) % 2, [0, 0], 2, 2, flags) == [0, 0, 0, 0]
+    for s in range(2):
+        assert J.set_phase_grating(GPU, s, pgr[s]) == 0
+    assert J.set_propagator(GPU, 0, pro) == 0
+    for i, (b0, b1) in enumerate(((0, 10), (20, 50))):
+        assert J.set_detector(GPU, i, *J.calc_ring_detector(b0, b1)) == 0
+    assert J.init_core(GPU) == 0
+    assert J.set_incident_wave(GPU, probe) == 0
+    return a
+
+
+def _launches(J, fuse, pos, npass, **kw):
+    J.L.JMS_SetPassFusion(fuse)
+    n0 = J.L.JMS_KernelLaunches()
+    e, out, ob = J.scan(pos, npass, **kw)
+    assert e == 0, e
+    return out, ob, J.L.JMS_KernelLaunches() - n0
+
+
+def _close(a, b, rel):
+    assert np.abs(b).max() > 0
+    assert np.abs(a.astype(np.float64) - b).max() <= rel * np.abs(b).max()
+
+
+@pytest.mark.parametrize("batch", [1, 8, 31])
+def test_a_smaller_batch_bounds_the_waves_of_a_launch(J, batch):
+    """A batch below the default is the caller's bound on the waves in flight: no batches are put together."""
+    a = _setup(J, 128)
+    pos = np.random.default_rng(2).uniform(0, a, (40, 2)).astype(np.float32)
+    J.L.JMS_SetScanBatch(batch)
+    varseq = np.zeros((1, 5), np.int32)
+    got, _, n1 = _launches(J, 1, pos, 1, varseq=varseq)
+    ref, _, n0 = _launches(J, 0, pos, 1, varseq=varseq)
+    assert n1 == n0, (n1, n0)
+    np.testing.assert_array_equal(got, ref)
