@@ -1168,9 +1168,10 @@ int JmsB200::ScanGPUDevice(int npos, const float* d_pos, float dz, int npass, co
 	// in configuration k.  Needs no plasmon paths and grating offsets within int
 	// range.  At most 4096 waves, which bounds the per-wave tables and sums.  A
 	// batch below the default is a caller's bound on the waves in flight: it is
-	// kept.
+	// kept.  So are the batches of a context with image, diffraction or wave
+	// channels, to which a launch of one wave adds.
 	constexpr long long kMergePoints = 1LL << 23, kMergeWaves = 4096;
-	const int Wm = B < kDefaultBatch ? B
+	const int Wm = B < kDefaultBatch || (imagedet_ & ~DET_INTEGRATED) ? B
 		: (int)std::max<long long>(B, std::min(kMergeWaves, kMergePoints / std::max(1LL, (long long)nx_ * ny_)));
 	const long long pool = slcoffset_.empty() ? 0
 		: slcoffset_.back() + (long long)nvarslc_.back() * npgx_ * npgy_;

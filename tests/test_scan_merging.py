@@ -70,3 +70,26 @@ def test_a_smaller_batch_bounds_the_waves_of_a_launch(J, batch):
     ref, _, n0 = _launches(J, 0, pos, 1, varseq=varseq)
     assert n1 == n0, (n1, n0)
     np.testing.assert_array_equal(got, ref)
+
+
+def test_channels_of_a_scan(J):
+    """A launch of one wave without a binned pattern adds to the context's channels; in a context that keeps any, the
+    scan's launches are those of its batches."""
+    flags = G.INT | G.DIF | G.IMG
+    n, nd = 64, 4
+    a = _setup(J, n, flags=flags)
+    pos = np.random.default_rng(4).uniform(0, a, (33, 2)).astype(np.float32)    # the last batch holds one position
+    varseq = np.random.default_rng(5).integers(0, 3, (2, 5)).astype(np.int32)
+    got = []
+    for fuse in (1, 0):
+        J.seed(3)
+        assert J.offset(GPU, 0.1, 0.2) == 0
+        assert J.gpu_multislice(0, 0, 1.0) == 0
+        assert J.num_det_planes() == nd
+        before = J.get_result(GPU, G.DIF, nd * n * n)
+        out, _, _ = _launches(J, fuse, pos, 2, varseq=varseq)
+        dif, img = J.get_result(GPU, G.DIF, nd * n * n), J.get_result(GPU, G.IMG, nd * n * n)
+        assert np.abs(dif - before).max() > 0
+        got.append((out, dif, img))
+    for x, y in zip(*got):
+        np.testing.assert_array_equal(x, y)
