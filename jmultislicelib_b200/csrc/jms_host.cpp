@@ -1190,10 +1190,6 @@ int JmsB200::ScanGPUDevice(int npos, const float* d_pos, float dz, int npass, co
 			drawn.resize((size_t)nbatch * npass * nobjslc_);
 			for (int k = 0; k < nbatch * npass; k++) GetRandomVariantSequence(drawn.data() + (size_t)k * nobjslc_);
 		}
-		// variants of position p in pass ip
-		auto variants = [&](int p, int ip) {
-			return varseq ? varseq + (size_t)ip * nobjslc_ : drawn.data() + ((size_t)(p / B) * npass + ip) * nobjslc_;
-		};
 		const int np_max = std::min(npos, Wm);      // positions per launch
 		const int kp = std::min(npass, std::max(1, Wm / np_max));
 		const size_t nw_max = (size_t)kp * np_max;
@@ -1214,15 +1210,21 @@ int JmsB200::ScanGPUDevice(int npos, const float* d_pos, float dz, int npass, co
 			for (int ip0 = 0; ip0 < npass; ip0 += kp) {
 				const int np = std::min(np_max, npos - p0), kk = std::min(kp, npass - ip0), nw = kk * np;
 				h_mulw_.assign((size_t)nw * nobjslc_, 0);
-				for (int k = 0; k < kk; k++)
-					for (int p = 0; p < np; p++) {
-						const int* var = variants(p0 + p, ip0 + k);
-						for (int j = 0; j < nobjslc_; j++) {
-							const int st = objslc_[j] % nscslc_;
-							h_mulw_[(size_t)j * nw + (size_t)k * np + p] =
-								(int)(slcoffset_[st] + (long long)var[j] * npgx_ * npgy_);
+				// one offset per slice and configuration, or per batch that drew its own
+				for (int j = 0; j < nobjslc_; j++) {
+					const int st = objslc_[j] % nscslc_;
+					for (int k = 0; k < kk; k++) {
+						int* row = &h_mulw_[(size_t)j * nw + (size_t)k * np];
+						for (int p = 0; p < np;) {
+							const int batch = (p0 + p) / B;
+							const int end = varseq ? np : std::min(np, (batch + 1) * B - p0);
+							const int v = varseq ? varseq[(size_t)(ip0 + k) * nobjslc_ + j]
+								: drawn[((size_t)batch * npass + ip0 + k) * nobjslc_ + j];
+							std::fill(row + p, row + end, (int)(slcoffset_[st] + (long long)v * npgx_ * npgy_));
+							p = end;
 						}
 					}
+				}
 				// stream order keeps the previous launch sequence's reads of the
 				// tables ahead of these writes
 				if (post(cudaMemcpyAsync(d_mulw_, h_mulw_.data(), sizeof(int) * h_mulw_.size(), cudaMemcpyHostToDevice,

@@ -93,3 +93,34 @@ def test_channels_of_a_scan(J):
         got.append((out, dif, img))
     for x, y in zip(*got):
         np.testing.assert_array_equal(x, y)
+
+
+@pytest.mark.parametrize("npos,npass", [(50, 5), (300, 2), (129, 3)])
+def test_uneven_groups(J, npos, npass):
+    """At 256^2 (128 waves a launch): configurations in groups of 2, 2, 1; positions in groups of 128, 128, 44 and of
+    128, 1, whose results lie past the first group's."""
+    a = _setup(J, 256)
+    rng = np.random.default_rng(npos)
+    pos = rng.uniform(0, a, (npos, 2)).astype(np.float32)
+    varseq = rng.integers(0, 3, (npass, 5)).astype(np.int32)
+    got, gb, n1 = _launches(J, 1, pos, npass, varseq=varseq, bin=4)
+    ref, rb, n0 = _launches(J, 0, pos, npass, varseq=varseq, bin=4)
+    assert n1 < n0
+    _close(got, ref, 2.0 ** -23)
+    _close(gb, rb, 1e-6)
+
+
+def test_draws_of_merged_batches(J):
+    """Without a variant sequence every batch of 32 positions draws its own configurations, in the order of the
+    sequential form, and leaves the generator where that form does."""
+    a = _setup(J, 256)
+    pos = np.random.default_rng(8).uniform(0, a, (50, 2)).astype(np.float32)
+    got = []
+    for fuse in (1, 0):
+        J.seed(21)
+        out, _, n = _launches(J, fuse, pos, 3)
+        nxt, _, _ = _launches(J, fuse, pos[:1], 1)
+        got.append((out, nxt, n))
+    assert got[0][2] < got[1][2]
+    _close(got[0][0], got[1][0], 2.0 ** -23)
+    np.testing.assert_array_equal(got[0][1], got[1][1])
