@@ -1024,7 +1024,7 @@ __device__ __forceinline__ void col_pass_tile(const PassArgs& p, int col0, const
 				v[e] = cmul(v[e], __ldg(mul + q), __ldg(mul1 + q));
 			}
 		}
-		int sx = p.plas_x, sy = p.plas_y, sx1 = 0, sy1 = 0;
+		int sx = p.plas_x, sy = p.plas_y, sx1 = NW == 2 ? sx : 0, sy1 = NW == 2 ? sy : 0;
 		if (p.plas_w) {
 			sx = __ldg(p.plas_w + 2 * b); sy = __ldg(p.plas_w + 2 * b + 1);
 			if constexpr (NW == 2) { sx1 = __ldg(p.plas_w + 2 * b1); sy1 = __ldg(p.plas_w + 2 * b1 + 1); }
