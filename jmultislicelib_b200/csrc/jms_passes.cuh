@@ -1111,11 +1111,14 @@ k_exit_cols(const PassArgs p)
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
 
 // chained: a pass kernel that waits for the one ahead of it itself (pass_wait)
-template <class K>
+template <class PL, class K>
 cudaError_t launch_k(K kern, dim3 grid, int threads, int smem, const PassArgs& p, cudaStream_t s, bool chained = false)
 {
 	static_assert(sizeof(PassArgs) < 4000, "kernel parameter block too large");
-	if (smem > 16 * 1024) {   // the default limit of 48 KB includes a kernel's static part
+	// the limit of 48 KB without this call includes a kernel's static part: at
+	// most the twiddle copy and the detector sums of 16 warps
+	constexpr int fixed = PL::TWS * (int)sizeof(float2) + 16 * 2 * kMaxDet * (int)sizeof(double);
+	if (smem + fixed > 48 * 1024) {
 		cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
 		if (e != cudaSuccess) return e;
 	}
@@ -1144,7 +1147,7 @@ cudaError_t launch_entry_t(const PassArgs& p, cudaStream_t s)
 {
 	constexpr int L = row_lines<PL>();
 	constexpr int smem = PL::template smem_elems<RowTileOf<PL>>() * (int)sizeof(V);
-	return launch_k(k_entry_rows<PL, V>, dim3((p.ny + L - 1) / L, wave_rows<V>(p)), L * PL::ROWT, smem, p, s);
+	return launch_k<PL>(k_entry_rows<PL, V>, dim3((p.ny + L - 1) / L, wave_rows<V>(p)), L * PL::ROWT, smem, p, s);
 }
 template <class PL, class V>
 cudaError_t launch_row_t(const PassArgs& p, cudaStream_t s)
@@ -1152,20 +1155,20 @@ cudaError_t launch_row_t(const PassArgs& p, cudaStream_t s)
 	constexpr int L = row_lines<PL>();
 	constexpr int smem = PL::template smem_elems<RowTileOf<PL>>() * (int)sizeof(V);
 	const dim3 grid((p.ny + L - 1) / L, wave_rows<V>(p));
-	if (p.plane >= 0) return launch_k(k_row_pass_read<PL, V>, grid, L * PL::ROWT, smem, p, s, true);
+	if (p.plane >= 0) return launch_k<PL>(k_row_pass_read<PL, V>, grid, L * PL::ROWT, smem, p, s, true);
 	if constexpr (Waves<V>::kN == 1 && PL::N >= 256) {
 		constexpr int LN = narrow_lines<PL>();
 		constexpr int smem_n = PL::template smem_elems<RowTile<LN, PL::ROWW>>() * (int)sizeof(V);
 		if ((long long)grid.x * p.nwave < kSMs)
-			return launch_k(k_row_pass<PL, V, LN>, dim3((p.ny + LN - 1) / LN, p.nwave), LN * PL::ROWT, smem_n, p, s, true);
+			return launch_k<PL>(k_row_pass<PL, V, LN>, dim3((p.ny + LN - 1) / LN, p.nwave), LN * PL::ROWT, smem_n, p, s, true);
 	}
-	return launch_k(k_row_pass<PL, V, L>, grid, L * PL::ROWT, smem, p, s, true);
+	return launch_k<PL>(k_row_pass<PL, V, L>, grid, L * PL::ROWT, smem, p, s, true);
 }
 template <class PL, class V, int C, bool READ, int NXC>
 cudaError_t launch_col_c(const PassArgs& p, cudaStream_t s)
 {
 	constexpr int smem = PL::template smem_elems<ColTile<C>>() * (int)sizeof(V);
-	return launch_k(k_col_pass<PL, V, C, READ, NXC>, dim3((p.nx + C - 1) / C, wave_rows<V>(p)), C * PL::TMAX, smem, p, s,
+	return launch_k<PL>(k_col_pass<PL, V, C, READ, NXC>, dim3((p.nx + C - 1) / C, wave_rows<V>(p)), C * PL::TMAX, smem, p, s,
 		true);
 }
 template <class PL, class V>
@@ -1188,7 +1191,7 @@ cudaError_t launch_exit_t(const PassArgs& p, cudaStream_t s)
 {
 	constexpr int C = PL::CC;
 	constexpr int smem = PL::template smem_elems<ColTile<C>>() * (int)sizeof(float2);
-	return launch_k(k_exit_cols<PL>, dim3((p.nx + C - 1) / C, p.nwave), C * PL::TMAX, smem, p, s);
+	return launch_k<PL>(k_exit_cols<PL>, dim3((p.nx + C - 1) / C, p.nwave), C * PL::TMAX, smem, p, s);
 }
 
 // The passes of a plan.  Wave pairs need the plan's values twice in registers:
