@@ -197,6 +197,8 @@ int JMS_ScanMultiFidelity(int ctx_full, int ctx_low, int npos, const float* pos,
 	const int* varseq, float* out_int);
 /* Kernel launches issued by the library so far. */
 long long JMS_KernelLaunches(void);
+/* Row and column pass launches so far that ran two waves per thread. */
+long long JMS_PairLaunches(void);
 /* Per-pass device timing: while on, each column and row pass launch is
  * bracketed by CUDA events on the library stream; JMS_PassTiming returns the
  * summed milliseconds and launch counts since the last JMS_SetPassTiming. */

@@ -80,7 +80,7 @@ SIGNATURES = {
     "JMS_ScanMultiFidelity": ([_i, _i, _i, _fp, _f, _i, _ip, _fp], _i),
     "JMS_GridSupported": ([_i, _i], _i),
     "JMS_SetPrecision": ([_i], _i), "JMS_GetPrecision": ([], _i), "JMS_TcStatus": ([], _i),
-    "JMS_TcLaunches": ([], C.c_longlong),
+    "JMS_TcLaunches": ([], C.c_longlong), "JMS_PairLaunches": ([], C.c_longlong),
     "JMS_ReadoutDetAvg": ([_i, _i, _fp, _fp], _i),
     "JMS_CreateContext": ([], _i), "JMS_SelectContext": ([_i], _i), "JMS_DestroyContext": ([_i], _i),
     "JMS_GraphBegin": ([_i, _ip], _i), "JMS_GraphEnd": ([], _i), "JMS_GraphLaunch": ([_i, _p, _i], _i),

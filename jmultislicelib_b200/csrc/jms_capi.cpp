@@ -286,6 +286,7 @@ int JMS_GridSupported(int nx, int ny) { return (jms::pass_supported(nx) && jms::
 int JMS_SetPrecision(int mode) { return J()->SetPrecision(mode); }
 int JMS_GetPrecision(void) { return J()->GetPrecision(); }
 int JMS_TcStatus(void) { return J()->TcStatus(); }
+long long JMS_PairLaunches(void) { return J()->PairLaunches(); }
 long long JMS_TcLaunches(void) { return J()->TcLaunches(); }
 
 int JMS_ReadoutDetAvg(int whichcode, int whichresult, float* dst, float* weight)

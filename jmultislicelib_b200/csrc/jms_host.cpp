@@ -609,13 +609,18 @@ int JmsB200::SetIncomingWaveGPU(const float* wav, bool bTranspose)
 	return 0;
 }
 
-// Wave pairs halve the CTAs of a launch, so they are taken where their column
-// tiles (8 columns of a pair) still reach every SM; results are the same bit
-// for bit either way.
+// Wave pairs halve the threads of a launch, so they are taken where single
+// waves would not all be resident at once: the GPU holds 1024 threads of the
+// single-wave passes per SM (64 registers), of 16 values each, 2.4 M points.
+// Slices of scans, single waves against pairs in us: 64^2 at 1.2 M points 8.8
+// against 11.5, 2.4 M 14.6 / 14.2, 4.8 M 25.8 / 23.2; 256^2 at 0.7 M 9.8 / 16.3,
+// 2.4 M 16.8 / 16.9, 7.2 M 42.7 / 38.7; 512^2 at 1.6 M 19.0 / 21.0, 2.6 M
+// 26.1 / 25.7, 7.3 M 59.9 / 52.9.  Results are the same bit for bit either way.
 bool JmsB200::use_pairs(int nwave) const
 {
+	constexpr long long kResident = 1024LL * 16 * kSMs;
 	return nwave > 1 && prec_ == 0 && prow_ && pcol_ && prow_->row2 && pcol_->col2 &&
-		(long long)((nwave + 1) / 2) * ((nx_ + 7) / 8) >= 148;
+		(long long)nwave * nx_ * ny_ >= kResident;
 }
 
 int JmsB200::ensure_work(int nwave)
@@ -758,6 +763,7 @@ int JmsB200::run_slices(int nwave, int islc0, const int* var, float weight, cons
 		else if (post((pairs ? prow_->row2 : prow_->row)(r, s), "GPUMultislice row pass")) return 601;
 		if (timing_on_) { ev_row_.push_back(timed_event()); cudaEventRecord(ev_row_.back(), s); }
 		launches_ += 2;
+		if (pairs) pair_launches_ += 2;
 	}
 	if (b_img && !pairs) { // exit plane image readout
 		PassArgs c = real;

@@ -174,6 +174,7 @@ public:
 	// 0, or 1 if a tensor-core pass reported an MMA wait that ran out (the
 	// flag is cleared by the call); synchronises the library stream
 	int TcStatus();
+	long long PairLaunches() const { return pair_launches_; }
 	long long TcLaunches() const { return tc_launches_; }
 	// device scratch of at least n doubles, owned by the context (grown on
 	// demand, freed with it); nullptr if the allocation fails
@@ -262,6 +263,7 @@ private:
 	int prec_ = 0;                  // 0 FP32, 1 BF16 hi+lo tensor core, 2 FP16 hi+lo tensor core
 	int* d_tcerr_ = nullptr;        // tensor-core pass status word
 	long long tc_launches_ = 0;
+	long long pair_launches_ = 0;    // pass launches over wave pairs
 	double* d_scratch_ = nullptr;
 	size_t scratch_cap_ = 0;
 	double* d_cv_ = nullptr;        // CvScratch: two halves of 2 n doubles

@@ -20,6 +20,7 @@
 
 namespace jms {
 
+constexpr int kSMs = 148;           // SMs of a B200
 constexpr int kMaxDet = 8;          // integrating detectors fused into one pass
 
 struct PassArgs {

@@ -922,7 +922,7 @@ __device__ __forceinline__ float2 plasmon_ramp(int sx, int sy, int x, int y, int
 // Columns per column-pass CTA: of single waves the plan's own, of wave pairs
 // half of it, so a CTA holds the same shared memory and half the threads; a
 // narrow tile where a launch would leave SMs idle.
-constexpr int kNarrow = 4, kSMs = 148;
+constexpr int kNarrow = 4;
 template <class PL, class V>
 __host__ __device__ constexpr int col_width(bool narrow)
 {

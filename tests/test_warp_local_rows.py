@@ -10,6 +10,9 @@ scan gives again.  A race between the lines of a CTA (one line's exchange
 writing into another line's region) shows up as a difference.  Every row plan
 of each length is run, on a specimen whose propagator has the 2/3 band gap (so
 warps of dead rows exit early), with readout planes (the readout row pass).
+One wave at a time leaves SMs idle, so long lines then take narrow tiles of
+rows and columns: the lengths without warp-local lines that have such tiles are
+among the sizes too, and every column plan is compared as well.
 """
 import numpy as np
 import pytest
@@ -22,6 +25,8 @@ GPU = 2
 # row plans with warp-local lines: 128 (8x16 pair), 192 (12x16), 240 (15x16),
 # 256 (16x16), 512 (16x32 pair), 768 (24x32), 1024 (32x32)
 SIZES = [128, 192, 240, 256, 512, 768, 1024]
+# further lengths whose single waves take narrow tiles
+NARROW = [320, 384, 480, 640, 720, 960, 2048]
 
 
 @pytest.fixture(scope="module")
@@ -55,26 +60,30 @@ def _setup(J, n, nobj=6, nvar=2, ndetper=3):
     return a, b, nobj
 
 
-@pytest.mark.parametrize("n", SIZES)
+@pytest.mark.parametrize("n", SIZES + NARROW)
 def test_batched_rows_equal_single_waves(J, n):
     a, b, nobj = _setup(J, n)
     pos = np.random.default_rng(n).uniform(0, a, (64, 2)).astype(np.float32)
     varseq = np.zeros((1, nobj), np.int32)
     nplan = J.L.JMS_PlanCount(n)
     try:
-        for ir in range(nplan):
-            assert J.L.JMS_SelectPlans(ir, 0) == 0
+        for ir, ic in [(k, 0) for k in range(nplan)] + [(0, k) for k in range(1, nplan)]:
+            assert J.L.JMS_SelectPlans(ir, ic) == 0
+            n0 = J.L.JMS_KernelLaunches()
             J.L.JMS_SetScanBatch(64)
             e, batched, _ = J.scan(pos, 1, varseq=varseq)
             assert e == 0, e
             e, again, _ = J.scan(pos, 1, varseq=varseq)
             assert e == 0, e
+            n1 = J.L.JMS_KernelLaunches()
             J.L.JMS_SetScanBatch(1)
             e, single, _ = J.scan(pos, 1, varseq=varseq)
             assert e == 0, e
+            # one launch sequence against one per position
+            assert J.L.JMS_KernelLaunches() - n1 > 60 * ((n1 - n0) // 2 - 2), (n0, n1)
             assert np.abs(batched).max() > 0
-            assert np.array_equal(batched, again), (n, ir)
-            assert np.array_equal(batched, single), (n, ir, np.abs(batched - single).max())
+            assert np.array_equal(batched, again), (n, ir, ic)
+            assert np.array_equal(batched, single), (n, ir, ic, np.abs(batched - single).max())
     finally:
         J.L.JMS_SetScanBatch(32)
         J.L.JMS_SelectPlans(0, 0)
