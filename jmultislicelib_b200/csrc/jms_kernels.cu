@@ -52,16 +52,17 @@ cudaError_t launch_cv_combine(double* out, const double* g1, const double* gm, l
 }
 
 // warp i = (position p, plane, detector) of n outputs; m = ndetslc * ndet
-// elements per wave; the waves of position p are p + k * step, k < nk.  The nk *
-// nblk terms go over the lanes, whose sums are added in a fixed order (one
-// thread walking them took 144 us for 16 x 64 terms of 2112 outputs: a chain of
-// dependent FP64 adds and loads).
+// elements per wave; the waves of position p are p + k * step, k < nk.  The nblk
+// terms of a wave go over the lanes, wave after wave, and the lanes' sums are
+// added in a fixed order (one thread walking all terms took 144 us for 16 x 64
+// terms of 2112 outputs: a chain of dependent FP64 adds and loads).
 __global__ void __launch_bounds__(256) k_finalize(const double* __restrict__ partial, int n, int m, int nblk, int step,
 	int nk, float weight, double* det_int)
 {
-	const int i = (blockIdx.x * 256 + threadIdx.x) / 32, lane = threadIdx.x & 31;
-	if (i >= n) return;
-	const int pos = i / m, e = i - pos * m;
+	const unsigned i = blockIdx.x * 8 + threadIdx.x / 32;
+	const int lane = threadIdx.x & 31;
+	if (i >= (unsigned)n) return;
+	const int pos = (int)i / m, e = (int)i - pos * m;
 	double s = 0.0;
 	for (int k = 0; k < nk; k++) {
 		const double* src = partial + ((long long)(pos + k * step) * m + e) * nblk;
