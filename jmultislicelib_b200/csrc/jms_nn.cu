@@ -25,8 +25,8 @@ __device__ __forceinline__ float bf(const __nv_bfloat16 v) { return __bfloat162f
 // in shared memory in one pass of independent loads per chunk of channels, and
 // keeps the reuse of a value in registers.  Batch 256, ten 16 x 16 channels, all
 // layers of a training step, against one thread per output (or per sum) reading
-// every operand from global memory: forward 92 -> 54 us, weight gradients
-// 152 -> 82, data gradients 102 -> 55; still mostly waiting on global loads.
+// every operand from global memory: forward 92 -> 53 us, weight gradients
+// 152 -> 80, data gradients 102 -> 51; still mostly waiting on global loads.
 // Every sum has one order of its FP32 additions, given at its kernel, that no
 // tile, chunk or grid changes: Adam divides a gradient by its own magnitude, so
 // in a few training steps another rounding of a gradient near zero becomes 1e-4
@@ -131,13 +131,11 @@ __global__ void __launch_bounds__(kNnThr) k_conv_bwd_data(const float* __restric
 					const int k = i / 64, h = i % 4;
 					const I pi = pix0 + (i / 4) % 16;
 					const int bi = (int)(pi / hw), ri = (int)(pi - (I)bi * hw), ai = ri / Wo + (h >> 1), di = ri % Wo + (h & 1);
-					float g = 0.f;
-					if (pi < npix && ai < Ho && di < Wo) {
-						const long long o = (((long long)bi * Co + k0 + k) * Ho + ai) * Wo + di;
-						g = dy[o];
-						if (relu && !(bf(y[o]) > 0.f)) g = 0.f;
-					}
-					gs[k][(i / 4) % 16][h] = g;
+					const bool in = pi < npix && ai < Ho && di < Wo;
+					const long long o = (((long long)bi * Co + k0 + k) * Ho + ai) * Wo + di;
+					const float g = in ? dy[o] : 0.f;
+					const __nv_bfloat16 yv = in && relu ? y[o] : __nv_bfloat16(1.f);
+					gs[k][(i / 4) % 16][h] = bf(yv) > 0.f ? g : 0.f;
 				}
 				#pragma unroll 12
 				for (int i = threadIdx.x; i < nk * 144; i += kNnThr) {
@@ -187,32 +185,34 @@ __global__ void __launch_bounds__(kNnThr) k_conv_bwd_data(const float* __restric
 }
 
 // dw[co][ci][ky][kx] = sum_b,oy,ox g[b][co][oy][ox] x[b][ci][iy][ix]; db[co] = sum g.
-// A CTA takes four output channels, one input channel and one row ky of taps: a
-// thread reads an output pixel's three taps once for the four channels, and the
-// three rows give the first layers, which have the most pixels and the fewest
-// channels, CTAs for every SM.  Four pixels' loads are in flight at once (first
-// layer 37 -> 26 us).  A sum runs over a thread's pixels (t, t + 256,
-// ...), then over the lanes of a warp in halves, then over the warps.  The CTAs
-// of ci = 0, ky = 1 also make db.
-constexpr int kBwCo = 4, kBwSums = 4 * kBwCo;
-template <class I>
+// A CTA takes NCO output channels, one input channel and one row ky of taps: a
+// thread reads an output pixel's three taps once for its channels.  Four channels
+// where that gives every SM two CTAs, else one: the first layers have the most
+// pixels and the fewest channels (1024 images of 3 x 64 x 64: 8.1 -> 1.1 ms for
+// the first layer with the next).  U pixels' loads are in flight at once, the
+// ReLU's outputs among them: loaded under a test of their own, each would be
+// waited for.  A sum runs over a thread's pixels (t, t + 256, ...),
+// then over the lanes of a warp in halves, then over the warps.  The CTAs of
+// ci = 0, ky = 1 also make db.
+template <class I, bool RELU, int NCO, int U>
 __global__ void __launch_bounds__(kNnThr) k_conv_bwd_weight(const __nv_bfloat16* __restrict__ x,
 	const float* __restrict__ dy, const __nv_bfloat16* __restrict__ y, float* __restrict__ dw, float* __restrict__ db,
-	int B, int Ci, int H, int W, int Co, int relu)
+	int B, int Ci, int H, int W, int Co)
 {
-	__shared__ float red[kNnThr / 32][kBwSums];
-	const int ci = blockIdx.x, co0 = blockIdx.y * kBwCo, ky = blockIdx.z;
+	constexpr int K = 4 * NCO;
+	__shared__ float red[kNnThr / 32][K];
+	const int ci = blockIdx.x, co0 = blockIdx.y * NCO, ky = blockIdx.z;
 	const int Ho = H / 2, Wo = W / 2, hw = Ho * Wo;
 	const I n = (I)B * hw;
-	float a[kBwSums];        // sum 4 c + kx of channel c, and 4 c + 3 its sum of g
+	float a[K];              // sum 4 c + kx of channel c, and 4 c + 3 its sum of g
 	#pragma unroll
-	for (int k = 0; k < kBwSums; k++) a[k] = 0.f;
+	for (int k = 0; k < K; k++) a[k] = 0.f;
 	// pixel (b, oy, ox) of i and its step of 256 pixels, carried instead of divided
 	int b = (int)threadIdx.x / hw, oy = (int)threadIdx.x % hw / Wo, ox = (int)threadIdx.x % hw % Wo;
 	const int sb = kNnThr / hw, sy = kNnThr % hw / Wo, sx = kNnThr % hw % Wo;
-	constexpr int U = 4;     // pixels whose loads are in flight together
 	for (I i = threadIdx.x; i < n; i += U * kNnThr) {
-		float v[U][3], g[U][kBwCo];
+		float v[U][3], g[U][NCO];
+		__nv_bfloat16 yv[RELU ? U : 1][NCO];
 		bool top[U], left[U], live[U];
 		#pragma unroll
 		for (int u = 0; u < U; u++) {
@@ -226,10 +226,10 @@ __global__ void __launch_bounds__(kNnThr) k_conv_bwd_weight(const __nv_bfloat16*
 			v[u][2] = top[u] ? bf(xp[2]) : 0.f;
 			const long long o = ((long long)b * Co + co0) * hw + p;
 			#pragma unroll
-			for (int c = 0; c < kBwCo; c++) {
+			for (int c = 0; c < NCO; c++) {
 				const bool in = live[u] && co0 + c < Co;
 				g[u][c] = in ? dy[o + (long long)c * hw] : 0.f;
-				if (relu && in && !(bf(y[o + (long long)c * hw]) > 0.f)) g[u][c] = 0.f;
+				if constexpr (RELU) yv[u][c] = in ? y[o + (long long)c * hw] : __nv_bfloat16(0.f);
 			}
 			ox += sx;
 			oy += sy + (ox >= Wo);
@@ -240,31 +240,32 @@ __global__ void __launch_bounds__(kNnThr) k_conv_bwd_weight(const __nv_bfloat16*
 		#pragma unroll
 		for (int u = 0; u < U; u++) {
 			#pragma unroll
-			for (int c = 0; c < kBwCo; c++) {
-				if (left[u]) a[4 * c] = fmaf(g[u][c], v[u][0], a[4 * c]);
-				if (top[u]) a[4 * c + 1] = fmaf(g[u][c], v[u][1], a[4 * c + 1]);
-				if (top[u]) a[4 * c + 2] = fmaf(g[u][c], v[u][2], a[4 * c + 2]);
-				if (live[u]) a[4 * c + 3] += g[u][c];
+			for (int c = 0; c < NCO; c++) {
+				const float gc = !RELU || bf(yv[RELU ? u : 0][c]) > 0.f ? g[u][c] : 0.f;
+				if (left[u]) a[4 * c] = fmaf(gc, v[u][0], a[4 * c]);
+				if (top[u]) a[4 * c + 1] = fmaf(gc, v[u][1], a[4 * c + 1]);
+				if (top[u]) a[4 * c + 2] = fmaf(gc, v[u][2], a[4 * c + 2]);
+				if (live[u]) a[4 * c + 3] += gc;
 			}
 		}
 	}
-	// 16 sums at once: each step halves the sums a lane holds, so lane 2 k ends
-	// with sum k
+	// all K sums at once: each step halves the sums a lane holds, until lane
+	// 32 / K k holds sum k
 	const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 	#pragma unroll
-	for (int h = 16; h > 1; h >>= 1) {
+	for (int h = 16, m = K / 2; h > 0; h >>= 1, m >>= 1) {
 		const bool up = lane & h;
 		#pragma unroll
-		for (int k = 0; k < h / 2; k++) {
-			const float keep = up ? a[k + h / 2] : a[k], send = up ? a[k] : a[k + h / 2];
+		for (int k = 0; k < m; k++) {
+			const float keep = up ? a[k + m] : a[k], send = up ? a[k] : a[k + m];
 			a[k] = keep + __shfl_xor_sync(0xffffffffu, send, h);
 		}
+		if (m == 0) a[0] += __shfl_xor_sync(0xffffffffu, a[0], h);
 	}
-	a[0] += __shfl_xor_sync(0xffffffffu, a[0], 1);
-	if (!(lane & 1)) red[warp][lane >> 1] = a[0];
+	if (lane % (32 / K) == 0) red[warp][lane / (32 / K)] = a[0];
 	__syncthreads();
 	const int k = threadIdx.x;
-	if (k >= kBwSums || co0 + k / 4 >= Co) return;
+	if (k >= K || co0 + k / 4 >= Co) return;
 	float s = 0.f;
 	#pragma unroll
 	for (int q = 0; q < kNnThr / 32; q++) s += red[q][k];
@@ -478,8 +479,16 @@ int JMS_NnConvBackward(const void* x, const void* w, const void* y, const float*
 	if (dx)
 		(big ? k_conv_bwd_data<long long> : k_conv_bwd_data<int>)<<<dim3((unsigned)((npix + 15) / 16), (unsigned)((Ci + 15) / 16)), kNnThr, 0, s>>>(dy,
 			(const __nv_bfloat16*)y, (const __nv_bfloat16*)w, dx, B, Ci, H, W, Co, relu);
-	(big ? k_conv_bwd_weight<long long> : k_conv_bwd_weight<int>)<<<dim3((unsigned)Ci, (unsigned)((Co + kBwCo - 1) / kBwCo), 3),
-		kNnThr, 0, s>>>((const __nv_bfloat16*)x, dy, (const __nv_bfloat16*)y, dw, db, B, Ci, H, W, Co, relu);
+	const bool many = 3LL * Ci * ((Co + 3) / 4) >= 296;
+	auto pick = [&](auto i) {
+		using I = decltype(i);
+		return relu ? (many ? k_conv_bwd_weight<I, true, 4, 4> : k_conv_bwd_weight<I, true, 1, 8>)
+			: (many ? k_conv_bwd_weight<I, false, 4, 4> : k_conv_bwd_weight<I, false, 1, 8>);
+	};
+	auto kern = big ? pick(0LL) : pick(0);
+	const unsigned nq = (unsigned)(many ? (Co + 3) / 4 : Co);
+	kern<<<dim3((unsigned)Ci, nq, 3), kNnThr, 0, s>>>((const __nv_bfloat16*)x, dy, (const __nv_bfloat16*)y, dw, db, B, Ci, H,
+		W, Co);
 	return ok(s);
 }
 
