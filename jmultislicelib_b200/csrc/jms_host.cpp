@@ -610,17 +610,15 @@ int JmsB200::SetIncomingWaveGPU(const float* wav, bool bTranspose)
 }
 
 // Wave pairs halve the threads of a launch, so they are taken where single
-// waves would not all be resident at once: the GPU holds 1024 threads of the
-// single-wave passes per SM (64 registers), of 16 values each, 2.4 M points.
+// waves would not all be resident at once (2.4 M points).
 // Slices of scans, single waves against pairs in us: 64^2 at 1.2 M points 8.8
 // against 11.5, 2.4 M 14.6 / 14.2, 4.8 M 25.8 / 23.2; 256^2 at 0.7 M 9.8 / 16.3,
 // 2.4 M 16.8 / 16.9, 7.2 M 42.7 / 38.7; 512^2 at 1.6 M 19.0 / 21.0, 2.6 M
 // 26.1 / 25.7, 7.3 M 59.9 / 52.9.  Results are the same bit for bit either way.
 bool JmsB200::use_pairs(int nwave) const
 {
-	constexpr long long kResident = 1024LL * 16 * kSMs;
 	return nwave > 1 && prec_ == 0 && prow_ && pcol_ && prow_->row2 && pcol_->col2 &&
-		(long long)nwave * nx_ * ny_ >= kResident;
+		(long long)nwave * nx_ * ny_ >= kResidentPoints;
 }
 
 int JmsB200::ensure_work(int nwave)

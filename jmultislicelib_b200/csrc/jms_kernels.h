@@ -21,6 +21,9 @@
 namespace jms {
 
 constexpr int kSMs = 148;           // SMs of a B200
+// points of single waves that are resident at once: 1024 threads per SM (64
+// registers) of 16 values
+constexpr long long kResidentPoints = 1024LL * 16 * kSMs;
 constexpr int kMaxDet = 8;          // integrating detectors fused into one pass
 
 struct PassArgs {

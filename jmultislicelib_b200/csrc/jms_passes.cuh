@@ -28,13 +28,14 @@
 // CTA barriers.  Stage twiddles come from a shared copy (TwShared).
 //
 // A launch of many waves holds two of them per thread (cpair, jms_fft.cuh) in
-// packed arithmetic: 59 thread instructions per element of the column pass
-// against 84 with one wave.  Per 512-wave launch at 512^2 the
-// column pass takes 424 us against 505, the row pass 278 against 311 (16 warps
-// of 128 registers per SM against 32 of 64).  Without its wave loads and stores
-// the column pass still takes 377 us (449 with single waves): it is bound by
-// on-chip work, FMA pipe, shared memory and issue each at about 60 %, not by
-// DRAM (222 us for its bytes).  Measured slower: 8 x 8 x 8 lines (589 / 510 us),
+// packed arithmetic: 61 thread instructions per element of the column pass
+// against 84 with one wave.  Per 512-wave launch at 512^2 the column pass takes
+// 424 us against 505, the row pass 278 against 311 (16 warps of 128 registers
+// per SM against 32 of 64).  No pipe is full: of a 256-wave launch (ncu) the
+// column pass keeps issue 44 %, FMA 46 %, shared memory 59 % and DRAM 31 % busy,
+// the row pass 45, 53, 74 and 53 %, and the longest stall of both is for global
+// loads.  The form before the early gratings took 377 of its 449 us without any
+// wave loads and stores.  Measured slower: 8 x 8 x 8 lines (589 / 510 us),
 // 4 or 16 columns of pairs per tile (476, 604), fewer registers with spills
 // (513, 649), and the halves of one line as a pair in place of two waves
 // (440 / 328).
@@ -763,8 +764,8 @@ k_entry_rows(const PassArgs p)
 // the variant with the readout code (used at readout planes only, as the
 // kernel k_row_pass_read with launch bounds of its own), so the steps without
 // readout do not carry its registers.
-// L rows per CTA.
-template <class PL, bool READ, class V, int L>
+// L rows per CTA.  FEW: single waves that are all resident at once (few_waves).
+template <class PL, bool READ, class V, int L, bool FEW>
 __device__ __forceinline__ void row_pass_body(const PassArgs& p)
 {
 	constexpr int N = PL::N, NT = L * PL::ROWT;
@@ -794,8 +795,8 @@ __device__ __forceinline__ void row_pass_body(const PassArgs& p)
 	const int yl = row0 + line;
 	const bool live = line < nval && j < PL::T && (yl <= p.row_k1 || yl >= p.row_k2);
 	// a launch of few single waves is a chain of latencies: the propagator is
-	// loaded ahead of the wait (pairs have no registers for it)
-	constexpr bool EARLY = Waves<V>::kN == 1 && !READ && PL::EMID <= 16;
+	// loaded ahead of the wait
+	constexpr bool EARLY = FEW && !READ && PL::EMID <= 16;
 	float2 w[EARLY ? PL::EMID : 1];
 	if constexpr (EARLY) {
 		int l2, pos;
@@ -879,20 +880,41 @@ template <class PL, class V>
 __host__ __device__ constexpr int row_blocks_sm(bool read)
 {
 	if (Waves<V>::kN == 2) return pair_min_blocks<row_threads<PL>()>();
-	return read ? read_min_blocks<PL>() : PL::RM <= 16 ? 0 : row_min_blocks<PL>();
+	return read ? read_min_blocks<PL>() : row_min_blocks<PL>();
 }
+// Single waves of plans of at most 16 values a thread have two forms.  Where all
+// waves of a launch are resident at once (kResidentPoints) it is a chain of
+// latencies, and the propagators or gratings are loaded ahead of the wait, which
+// takes 80 to 100 registers; a larger launch keeps to 64, since it needs the
+// CTAs.  Us a slice, early loads against 64 registers: 64^2, 73 waves 5.0
+// against 7.5, 192^2, 32 waves 10.8 / 14.1, 240^2, 27 waves 12.9 / 17.2, 256^2,
+// 18 waves 9.5 / 13.8, 36 waves 16.8 / 17.2; 1024 x 512, 64 waves (512-point
+// columns, one CTA per SM in place of two) 300 / 240.
+inline bool few_waves(const PassArgs& p) { return (long long)p.nwave * p.nx * p.ny < kResidentPoints; }
+// Narrow tiles (4 columns, or rows for about 64 threads) in place of ctas full
+// ones: for lines of 256 or more up to 16 values a thread where the full tiles
+// do not reach every SM (512^2, us a slice with full rows and columns, narrow
+// rows, both narrow: one wave 12.6, 14.0, 11.0; four 19.7, 17.5, 16.6), for
+// longer ones from 480 on where they leave a third of the SMs idle (480^2, one
+// wave 12.9 / 12.1, 768^2 18.6 / 17.5; but 320^2 8.3 / 9.4, 384^2, two waves
+// 10.1 / 13.2, 1024^2 22.1 / 23.1).
+template <class PL>
+constexpr bool has_narrow() { return PL::N >= (PL::RM <= 16 ? 256 : 480); }
+template <class PL>
+constexpr bool use_narrow(long long ctas) { return PL::RM <= 16 ? ctas < kSMs : 3 * ctas <= 2 * kSMs; }
+constexpr int kNarrow = 4;
 // plain row pass; the readout planes use k_row_pass_read
-template <class PL, class V, int L>
-__global__ void __launch_bounds__(L * PL::ROWT, L == row_lines<PL>() ? row_blocks_sm<PL, V>(false) : 0)
+template <class PL, class V, int L, bool FEW>
+__global__ void __launch_bounds__(L * PL::ROWT, FEW ? 0 : row_blocks_sm<PL, V>(false))
 k_row_pass(const PassArgs p)
 {
-	row_pass_body<PL, false, V, L>(p);
+	row_pass_body<PL, false, V, L, FEW>(p);
 }
-template <class PL, class V>
-__global__ void __launch_bounds__(row_threads<PL>(), row_blocks_sm<PL, V>(true))
+template <class PL, class V, bool FEW>
+__global__ void __launch_bounds__(row_threads<PL>(), FEW ? 0 : row_blocks_sm<PL, V>(true))
 k_row_pass_read(const PassArgs p)
 {
-	row_pass_body<PL, true, V, row_lines<PL>()>(p);
+	row_pass_body<PL, true, V, row_lines<PL>(), FEW>(p);
 }
 
 // Live rows of a column-pass thread as a bit mask: bit m is set when row
@@ -922,7 +944,6 @@ __device__ __forceinline__ float2 plasmon_ramp(int sx, int sy, int x, int y, int
 // Columns per column-pass CTA: of single waves the plan's own, of wave pairs
 // half of it, so a CTA holds the same shared memory and half the threads; a
 // narrow tile where a launch would leave SMs idle.
-constexpr int kNarrow = 4;
 template <class PL, class V>
 __host__ __device__ constexpr int col_width(bool narrow)
 {
@@ -939,12 +960,14 @@ __host__ __device__ constexpr int col_width(bool narrow)
 // Up to 16 grating values a thread are loaded into registers early: for wave
 // pairs and plans of more values before the second DFT, whose arithmetic hides
 // the loads' latency (512^2 pairs, 512 waves: 449 -> 424 us; 1024^2, 128 waves:
-// 533 -> 503 us), for other single waves ahead of everything else.
-template <class PL, class V, int C, bool READ, int NXC, bool SYNC, class TW>
+// 533 -> 503 us), for other single waves in launches of few (FEW) ahead of
+// everything else.
+template <class PL, class V, int C, bool READ, int NXC, bool FEW, bool SYNC, class TW>
 __device__ __forceinline__ void col_pass_tile(const PassArgs& p, int col0, const TW& tw, V* sm)
 {
 	constexpr int NW = Waves<V>::kN;
-	constexpr int PRE = READ ? 0 : PL::EMID <= 16 ? PL::EMID : 16;   // values loaded early
+	// values loaded early
+	constexpr int PRE = READ || (NW == 1 && PL::EMID <= 16 && !FEW) ? 0 : PL::EMID <= 16 ? PL::EMID : 16;
 	constexpr bool EARLY = PRE > 0;
 	static_assert(!(READ && NW == 2), "images are read out of single waves only");
 	using T = ColTile<C>;
@@ -976,7 +999,7 @@ __device__ __forceinline__ void col_pass_tile(const PassArgs& p, int col0, const
 			}
 		}
 	};
-	if constexpr (NW == 1 && PL::EMID <= 16) load_t();   // single waves: ahead of the wait
+	if constexpr (NW == 1 && PL::EMID <= 16) load_t();   // few single waves: ahead of the wait
 	pass_wait();
 	// 32-bit offsets within a wave (nx * ny < 2^31): one base pointer per
 	// thread and a row stride, instead of a 64-bit product per element
@@ -1050,17 +1073,17 @@ __device__ __forceinline__ void col_pass_tile(const PassArgs& p, int col0, const
 	}
 }
 
-// Resident CTAs asked of a column pass: wave pairs at most 128 registers;
-// single waves of the full width as the row pass; narrow tiles are few and free.
+// Resident CTAs asked of a column pass: wave pairs at most 128 registers; many
+// single waves as the row pass; few are free.
 template <class PL, class V, int C>
-__host__ __device__ constexpr int col_blocks_sm(bool read)
+__host__ __device__ constexpr int col_blocks_sm(bool read, bool few)
 {
 	constexpr int NT = C * PL::TMAX;
 	if (Waves<V>::kN == 2) return pair_min_blocks<NT>();
-	return PL::RM > 16 && !read ? pass_min_blocks<PL, NT>() : 0;
+	return read || (few && PL::RM <= 16) ? 0 : pass_min_blocks<PL, NT>();
 }
-template <class PL, class V, int C, bool READ, int NXC>
-__global__ void __launch_bounds__(C * PL::TMAX, col_blocks_sm<PL, V, C>(READ))
+template <class PL, class V, int C, bool READ, int NXC, bool FEW>
+__global__ void __launch_bounds__(C * PL::TMAX, col_blocks_sm<PL, V, C>(READ, FEW))
 k_col_pass(const PassArgs p)
 {
 	pass_trigger();
@@ -1068,9 +1091,9 @@ k_col_pass(const PassArgs p)
 	__shared__ float2 tws[PL::TWS];
 	if constexpr (PL::SMEM_TW) {
 		fill_tw_shared<PL::A, PL::B, PL::ROW, C * PL::TMAX>(tws, p.twy, threadIdx.x);   // barrier after the wave loads
-		col_pass_tile<PL, V, C, READ, NXC, true>(p, blockIdx.x * C, TwShared<PL::ROW>{tws}, sm);
+		col_pass_tile<PL, V, C, READ, NXC, FEW, true>(p, blockIdx.x * C, TwShared<PL::ROW>{tws}, sm);
 	}
-	else col_pass_tile<PL, V, C, READ, NXC, false>(p, blockIdx.x * C, TwGlobal{p.twy}, sm);
+	else col_pass_tile<PL, V, C, READ, NXC, FEW, false>(p, blockIdx.x * C, TwGlobal{p.twy}, sm);
 }
 
 // Exit column pass: IFT_y -> real-space readout (plane), no store.
@@ -1155,36 +1178,49 @@ cudaError_t launch_row_t(const PassArgs& p, cudaStream_t s)
 	constexpr int L = row_lines<PL>();
 	constexpr int smem = PL::template smem_elems<RowTileOf<PL>>() * (int)sizeof(V);
 	const dim3 grid((p.ny + L - 1) / L, wave_rows<V>(p));
-	if (p.plane >= 0) return launch_k<PL>(k_row_pass_read<PL, V>, grid, L * PL::ROWT, smem, p, s, true);
-	if constexpr (Waves<V>::kN == 1 && PL::N >= 256) {
-		constexpr int LN = narrow_lines<PL>();
-		constexpr int smem_n = PL::template smem_elems<RowTile<LN, PL::ROWW>>() * (int)sizeof(V);
-		if ((long long)grid.x * p.nwave < kSMs)
-			return launch_k<PL>(k_row_pass<PL, V, LN>, dim3((p.ny + LN - 1) / LN, p.nwave), LN * PL::ROWT, smem_n, p, s, true);
+	if (p.plane >= 0) {
+		// held to 64 registers the readout spills: few waves need not be
+		if constexpr (Waves<V>::kN == 1 && PL::RM <= 16)
+			if (few_waves(p)) return launch_k<PL>(k_row_pass_read<PL, V, true>, grid, L * PL::ROWT, smem, p, s, true);
+		return launch_k<PL>(k_row_pass_read<PL, V, false>, grid, L * PL::ROWT, smem, p, s, true);
 	}
-	return launch_k<PL>(k_row_pass<PL, V, L>, grid, L * PL::ROWT, smem, p, s, true);
+	if constexpr (Waves<V>::kN == 1) {
+		if constexpr (has_narrow<PL>()) {
+			constexpr int LN = narrow_lines<PL>();
+			constexpr int smem_n = PL::template smem_elems<RowTile<LN, PL::ROWW>>() * (int)sizeof(V);
+			if (use_narrow<PL>((long long)grid.x * p.nwave))
+				return launch_k<PL>(k_row_pass<PL, V, LN, true>, dim3((p.ny + LN - 1) / LN, p.nwave), LN * PL::ROWT, smem_n, p, s, true);
+		}
+		if constexpr (PL::RM <= 16)
+			if (few_waves(p)) return launch_k<PL>(k_row_pass<PL, V, L, true>, grid, L * PL::ROWT, smem, p, s, true);
+	}
+	return launch_k<PL>(k_row_pass<PL, V, L, false>, grid, L * PL::ROWT, smem, p, s, true);
 }
-template <class PL, class V, int C, bool READ, int NXC>
+template <class PL, class V, int C, bool READ, int NXC, bool FEW>
 cudaError_t launch_col_c(const PassArgs& p, cudaStream_t s)
 {
 	constexpr int smem = PL::template smem_elems<ColTile<C>>() * (int)sizeof(V);
-	return launch_k<PL>(k_col_pass<PL, V, C, READ, NXC>, dim3((p.nx + C - 1) / C, wave_rows<V>(p)), C * PL::TMAX, smem, p, s,
+	return launch_k<PL>(k_col_pass<PL, V, C, READ, NXC, FEW>, dim3((p.nx + C - 1) / C, wave_rows<V>(p)), C * PL::TMAX, smem, p, s,
 		true);
 }
 template <class PL, class V>
 cudaError_t launch_col_t(const PassArgs& p, cudaStream_t s)
 {
-	constexpr int C = col_width<PL, V>(false), CN = col_width<PL, V>(true);
+	constexpr int C = col_width<PL, V>(false), CN = col_width<PL, V>(true), N = PL::N;
+	const bool square = p.nx == N;
 	if constexpr (Waves<V>::kN == 1) {
 		if (p.plane >= 0)
-			return p.nx == PL::N ? launch_col_c<PL, V, C, true, PL::N>(p, s) : launch_col_c<PL, V, C, true, 0>(p, s);
-		// fewer tiles than SMs: narrow tiles, for lines long enough to fill
-		// their warps (one wave: 512^2 7.1 -> 5.4 us per launch, 256^2 4.5
-		// either way, 64^2 2.5 -> 3.3)
-		if constexpr (PL::N >= 320)
-			if ((long long)((p.nx + C - 1) / C) * p.nwave < kSMs) return launch_col_c<PL, V, CN, false, 0>(p, s);
+			return square ? launch_col_c<PL, V, C, true, N, false>(p, s) : launch_col_c<PL, V, C, true, 0, false>(p, s);
+		// 256-point columns gain nothing by narrow tiles (4.5 us either way)
+		if constexpr (has_narrow<PL>() && N >= 320) {
+			if (use_narrow<PL>((long long)((p.nx + C - 1) / C) * p.nwave)) return launch_col_c<PL, V, CN, false, 0, true>(p, s);
+		}
+		else if constexpr (PL::RM <= 16) {
+			if (few_waves(p))
+				return square ? launch_col_c<PL, V, C, false, N, true>(p, s) : launch_col_c<PL, V, C, false, 0, true>(p, s);
+		}
 	}
-	return p.nx == PL::N ? launch_col_c<PL, V, C, false, PL::N>(p, s) : launch_col_c<PL, V, C, false, 0>(p, s);
+	return square ? launch_col_c<PL, V, C, false, N, false>(p, s) : launch_col_c<PL, V, C, false, 0, false>(p, s);
 }
 template <class PL>
 cudaError_t launch_exit_t(const PassArgs& p, cudaStream_t s)

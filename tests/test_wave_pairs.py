@@ -63,6 +63,10 @@ def _setup(J, nx, ny, nobj, nvar, npg=None):
     # a long axis; row lines rounded up to 32 threads, and of two warps: no pairs, but lines that run by themselves
     (320, 160, 9, 1, None), (720, 48, 40, 1, None), (480, 64, 40, 1, None), (384, 48, 40, 1, None),
     (2048, 64, 12, 1, None),
+    # a long axis in a launch too large for the other axis's passes to load their operands early
+    (1024, 512, 7, 1, None), (512, 1024, 7, 1, None), (768, 256, 13, 1, None), (256, 768, 13, 1, None),
+    (640, 192, 20, 1, None), (192, 640, 20, 1, None), (480, 240, 22, 1, None), (240, 480, 22, 1, None),
+    (320, 128, 61, 1, None), (128, 320, 61, 1, None), (1024, 64, 38, 1, None), (64, 1024, 38, 1, None),
     # from the fewest waves that take pairs on
     (512, 512, 5, 2, None), (512, 512, 11, 1, None), (512, 256, 7, 3, None), (256, 256, 37, 1, None),
     (256, 192, 1, 51, None), (192, 240, 53, 1, None), (128, 128, 51, 3, None), (128, 64, 297, 1, (64, 32)),
