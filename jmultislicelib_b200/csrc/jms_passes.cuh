@@ -572,14 +572,14 @@ __device__ __forceinline__ void readout_bin(const PassArgs& p, int b, int y, int
 
 // Fourier-space readout of a row tile: thread (y, live) holds the E values v of
 // row y at columns kx_of(e); b0 is the (first) wave.  Called by every thread
-// of the CTA.
-template <int NT, int E, class V, int RM, class KX>
+// of the CTA.  CHAN: with the channels of a single wave, whose loads in flight
+// take 114 registers at 512 points (without them it is 64, and none spills).
+template <bool CHAN, int NT, int E, class V, int RM, class KX>
 __device__ __forceinline__ void readout_rows(const PassArgs& p, int b0, int y, bool live, const V (&v)[RM], const KX& kx_of)
 {
 	constexpr int NW = Waves<V>::kN;
-	// channels in loops of their own (uniform tests), so their registers do
-	// not add to those of the other loads
-	if constexpr (NW == 1) {
+	// channels in loops of their own (uniform tests)
+	if constexpr (CHAN && NW == 1) {
 		if ((p.dif || p.dif_avg || p.wff || p.wff_avg) && live) {
 			// diffraction and wave channels (ReadoutDifDet_d, src/JMultiSlice.cpp:4277-4359)
 			const long long c = (long long)b0 * p.chan_wstride + (long long)p.plane * p.nx * p.ny;
@@ -749,7 +749,7 @@ k_entry_rows(const PassArgs p)
 			else v[m] = load_v(W + (long long)y * N + kx);
 		}
 	}
-	if (p.plane >= 0) readout_rows<NT, PL::A>(p, b, y, live, v, [&](int m) { return j + PL::B * m; });
+	if (p.plane >= 0) readout_rows<true, NT, PL::A>(p, b, y, live, v, [&](int m) { return j + PL::B * m; });
 	PL::template to_mid<true, T>(v, sm, TwGlobal{p.twx}, tid);
 	int pos;
 	T::template role<PL::TMID>(tid, line, pos);
@@ -765,7 +765,8 @@ k_entry_rows(const PassArgs p)
 // kernel k_row_pass_read with launch bounds of its own), so the steps without
 // readout do not carry its registers.
 // L rows per CTA.  FEW: single waves that are all resident at once (few_waves).
-template <class PL, bool READ, class V, int L, bool FEW>
+// CHAN: the readout adds to channels too.
+template <class PL, bool READ, class V, int L, bool FEW, bool CHAN>
 __device__ __forceinline__ void row_pass_body(const PassArgs& p)
 {
 	constexpr int N = PL::N, NT = L * PL::ROWT;
@@ -839,7 +840,7 @@ __device__ __forceinline__ void row_pass_body(const PassArgs& p)
 			}
 		}
 		if constexpr (READ)
-			readout_rows<NT, PL::EMID>(p, blockIdx.y * Waves<V>::kN, y, mid_live, v,
+			readout_rows<CHAN, NT, PL::EMID>(p, blockIdx.y * Waves<V>::kN, y, mid_live, v,
 				[&](int e) { return PL::mid(pos, e); });
 	}
 	if (!p.store) return;
@@ -908,13 +909,13 @@ template <class PL, class V, int L, bool FEW>
 __global__ void __launch_bounds__(L * PL::ROWT, FEW ? 0 : row_blocks_sm<PL, V>(false))
 k_row_pass(const PassArgs p)
 {
-	row_pass_body<PL, false, V, L, FEW>(p);
+	row_pass_body<PL, false, V, L, FEW, false>(p);
 }
-template <class PL, class V, bool FEW>
-__global__ void __launch_bounds__(row_threads<PL>(), FEW ? 0 : row_blocks_sm<PL, V>(true))
+template <class PL, class V, bool CHAN>
+__global__ void __launch_bounds__(row_threads<PL>(), CHAN ? 0 : row_blocks_sm<PL, V>(true))
 k_row_pass_read(const PassArgs p)
 {
-	row_pass_body<PL, true, V, row_lines<PL>(), FEW>(p);
+	row_pass_body<PL, true, V, row_lines<PL>(), false, CHAN>(p);
 }
 
 // Live rows of a column-pass thread as a bit mask: bit m is set when row
@@ -1179,9 +1180,19 @@ cudaError_t launch_row_t(const PassArgs& p, cudaStream_t s)
 	constexpr int smem = PL::template smem_elems<RowTileOf<PL>>() * (int)sizeof(V);
 	const dim3 grid((p.ny + L - 1) / L, wave_rows<V>(p));
 	if (p.plane >= 0) {
-		// held to 64 registers the readout spills: few waves need not be
-		if constexpr (Waves<V>::kN == 1 && PL::RM <= 16)
-			if (few_waves(p)) return launch_k<PL>(k_row_pass_read<PL, V, true>, grid, L * PL::ROWT, smem, p, s, true);
+		// Channels come with runs of one wave.  Plans of at most 16 values take
+		// that form for few waves too: its registers keep all of a detector's
+		// loads in flight, and two CTAs are resident on an SM.  Us a slice with a
+		// readout in each, against the form without channels: 512^2, four waves
+		// (170 CTAs of live rows) 19.6 / 25.2, six (255) 21.6 / 26.2, eight (341)
+		// 28.1 / 26.7; 256^2, 24 waves (256) 18.1 / 22.0, 32 (341) 25.7 / 23.4.
+		if constexpr (Waves<V>::kN == 1) {
+			const int gap = p.row_k2 - p.row_k1 - 1;      // rows of the propagator's band gap
+			const long long live = gap > 0 && gap < p.ny ? p.ny - gap : p.ny;
+			if (p.dif || p.dif_avg || p.wff || p.wff_avg ||
+				(PL::RM <= 16 && (long long)grid.x * p.nwave * live <= 2LL * kSMs * p.ny))
+				return launch_k<PL>(k_row_pass_read<PL, V, true>, grid, L * PL::ROWT, smem, p, s, true);
+		}
 		return launch_k<PL>(k_row_pass_read<PL, V, false>, grid, L * PL::ROWT, smem, p, s, true);
 	}
 	if constexpr (Waves<V>::kN == 1) {
