@@ -155,7 +155,10 @@ int JMS_ScanGPUDevice(int npos, const float* d_pos, float dz, int npass, const i
 /* Probe positions processed together in one pass sequence (default 32).  With
  * pass fusion on and a batch of at least the default, scans of small grids put
  * more waves into a launch, up to 64 MB of them and 4096; a smaller batch
- * bounds the waves in flight. */
+ * bounds the waves in flight.  A launch of one wave without a binned pattern
+ * also adds to the context's image, diffraction and wave channels, as a run of
+ * GPUMultislice does but without its averaging weight; a context that has such
+ * channels keeps its batches. */
 int JMS_SetScanBatch(int nwave);
 /* Frozen-phonon configurations in one launch (no counterpart in the
  * reference, whose GPUMultislice runs one wave per call,
@@ -165,7 +168,7 @@ int JMS_SetScanBatch(int nwave);
  * library draws all configurations first, in the sequential order): each
  * wave reads its own configuration's grating, and the detector sums and
  * binned patterns of a position collect its waves in a fixed order.  on = 1
- * (default) allows it, 0 runs one launch sequence per configuration.  Scans
+ * (default) allows it, 0 runs one launch sequence per batch and configuration.  Scans
  * enqueued during a stream capture always take the sequential form. */
 int JMS_SetPassFusion(int on);
 /* Multi-fidelity frozen-phonon scan (no counterpart in the reference, which

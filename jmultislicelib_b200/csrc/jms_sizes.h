@@ -1,11 +1,11 @@
 // jms_sizes.h -- supported line lengths and the candidate line plans of each
-// (jms_passes.cuh).  Plan<A, B, C> splits N = A * B (A, B <= 32, radices 2, 3,
-// 4, 5; paired threads when B = 2A); Plan3<R, C> runs N = R^3 in three stages;
+// (jms_passes.cuh).  Plan<A, B, C> splits N = A * B (A <= 32, B <= 64, radices 2,
+// 3, 4, 5; paired threads when B = 2A); Plan3<R, C> runs N = R^3 in three stages;
 // C is the column-pass tile width: 8 columns for plans of more than 16 values a
 // thread, whose wider tiles leave an SM one CTA (per 512 or 256 waves, c16 -> c8:
 // 320 291 -> 219 us, 384 388 -> 357, 480 605 -> 545, 640 514 -> 458, 720 631 -> 586,
 // 768 660 -> 598, 960 545 -> 477, 1024 570 -> 503).  The first plan of a length is its default;
-// JMS_Autotune picks among the candidates by timing them (jms_tune.cpp).
+// JMS_Autotune picks among the candidates by timing them (jms_host.cpp).
 #pragma once
 #include "jms_kernels.h"
 
