@@ -12,6 +12,7 @@
 // Layouts: activations [B][C][H][W]; conv weights [Co][Ci][3][3]; linear
 // weights [O][C].  The ReLU mask of a layer is its stored output (y > 0).
 #include "../../include/jms_b200.h"
+#include "jms_kernels.h"
 
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
@@ -461,7 +462,7 @@ int JMS_NnConvForward(const void* x, const void* w, const float* bias, void* y, 
 	// else 16-pixel tiles
 	const long long npix = (long long)B * (H / 2) * (W / 2);
 	const unsigned ncg = (unsigned)((Co + 15) / 16);
-	const bool wide = (npix + 63) / 64 * ncg >= 148;
+	const bool wide = (npix + 63) / 64 * ncg >= jms::kSMs;
 	const long long tile = wide ? 64 : 16;
 	auto kern = npix > kMaxPix32 ? k_conv_fwd<64, long long> : wide ? k_conv_fwd<64, int> : k_conv_fwd<16, int>;
 	kern<<<dim3((unsigned)((npix + tile - 1) / tile), ncg), kNnThr, 0, s>>>((const __nv_bfloat16*)x,
@@ -479,7 +480,7 @@ int JMS_NnConvBackward(const void* x, const void* w, const void* y, const float*
 	if (dx)
 		(big ? k_conv_bwd_data<long long> : k_conv_bwd_data<int>)<<<dim3((unsigned)((npix + 15) / 16), (unsigned)((Ci + 15) / 16)), kNnThr, 0, s>>>(dy,
 			(const __nv_bfloat16*)y, (const __nv_bfloat16*)w, dx, B, Ci, H, W, Co, relu);
-	const bool many = 3LL * Ci * ((Co + 3) / 4) >= 296;
+	const bool many = 3LL * Ci * ((Co + 3) / 4) >= 2 * jms::kSMs;
 	auto pick = [&](auto i) {
 		using I = decltype(i);
 		return relu ? (many ? k_conv_bwd_weight<I, true, 4, 4> : k_conv_bwd_weight<I, true, 1, 8>)
